@@ -608,52 +608,59 @@ sparse_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
   }
 }
 
-// Merges the partial results of split lists: one CTA per group, one thread per tile row.
+// Merges the partial results of split lists.
 //   out = sum_i O_i 2^(m_i - M) / sum_i l_i 2^(m_i - M),  M = max_i m_i
+// Bound by the latency of its loads from L2 (parts of 33 KB, a few MB per layer), so the rows of a group are
+// spread over kMergeCtas CTAs, eight threads per row with eight columns each, and every thread has four parts
+// in flight.  One sequence of 16384 tokens (12 heads, 12 groups of 20-odd parts), attention + merge: 73 us, with
+// one CTA per group and one thread per row 115 us.
+constexpr int kMergeCtas = 8;
+constexpr int kMergeRows = 128 / kMergeCtas;
 template <bool BF16>
-__global__ void __launch_bounds__(128) merge_partials_kernel(uint16_t* __restrict__ ctx,
-                                                             const int32_t* __restrict__ groups,
-                                                             const float* __restrict__ part_o,
-                                                             const float* __restrict__ part_ml, int hidden) {
+__global__ void __launch_bounds__(8 * kMergeRows) merge_partials_kernel(uint16_t* __restrict__ ctx,
+                                                                        const int32_t* __restrict__ groups,
+                                                                        const float* __restrict__ part_o,
+                                                                        const float* __restrict__ part_ml, int hidden) {
   RT_PDL_LAUNCH_DEPENDENTS();
   RT_PDL_WAIT();
   const int32_t* g = groups + blockIdx.x * 6;
   const int first = g[0], parts = g[1], head = g[4] & 255;
-  const int row = threadIdx.x;
+  const int row = blockIdx.y * kMergeRows + (threadIdx.x >> 3);
+  const int col = (threadIdx.x & 7) * 8;
   const int tok0 = row < 64 ? g[2] : g[3];
   if (tok0 < 0) return;
+  const float2* ml = reinterpret_cast<const float2*>(part_ml) + static_cast<size_t>(first) * 128 + row;
+  const float* src = part_o + (static_cast<size_t>(first) * 128 + row) * 64 + col;
   float M = -INFINITY;
-  for (int i = 0; i < parts; ++i) M = fmaxf(M, part_ml[(static_cast<size_t>(first + i) * 128 + row) * 2]);
+#pragma unroll 4
+  for (int i = 0; i < parts; ++i) M = fmaxf(M, ml[i * 128].x);
   float L = 0.f;
+  float acc[8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) acc[k] = 0.f;
+#pragma unroll 4
   for (int i = 0; i < parts; ++i) {
-    const float2 ml = *reinterpret_cast<const float2*>(part_ml + (static_cast<size_t>(first + i) * 128 + row) * 2);
-    L += ml.y * ex2(ml.x - M);
+    const float2 v = ml[i * 128];
+    const float4 a = *reinterpret_cast<const float4*>(src + static_cast<size_t>(i) * 128 * 64);
+    const float4 b = *reinterpret_cast<const float4*>(src + static_cast<size_t>(i) * 128 * 64 + 4);
+    const float w = ex2(v.x - M);
+    L += v.y * w;
+    acc[0] += w * a.x;
+    acc[1] += w * a.y;
+    acc[2] += w * a.z;
+    acc[3] += w * a.w;
+    acc[4] += w * b.x;
+    acc[5] += w * b.y;
+    acc[6] += w * b.z;
+    acc[7] += w * b.w;
   }
   const float inv = 1.0f / L;
-  uint16_t* dst = ctx + static_cast<size_t>(tok0 + (row & 63)) * hidden + head * 64;
-#pragma unroll 1
-  for (int c = 0; c < 64; c += 16) {
-    float acc[16];
-#pragma unroll
-    for (int k = 0; k < 16; ++k) acc[k] = 0.f;
-    for (int i = 0; i < parts; ++i) {
-      const size_t base = static_cast<size_t>(first + i) * 128 + row;
-      const float w = ex2(part_ml[base * 2] - M);
-      const float4* src = reinterpret_cast<const float4*>(part_o + base * 64 + c);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const float4 v = src[q];
-        acc[4 * q] += w * v.x;
-        acc[4 * q + 1] += w * v.y;
-        acc[4 * q + 2] += w * v.z;
-        acc[4 * q + 3] += w * v.w;
-      }
-    }
-    uint32_t o[8];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) o[k] = pack2<BF16>(acc[2 * k] * inv, acc[2 * k + 1] * inv);
-    st_global_v8(dst + c, o);
-  }
+  uint4 o;
+  o.x = pack2<BF16>(acc[0] * inv, acc[1] * inv);
+  o.y = pack2<BF16>(acc[2] * inv, acc[3] * inv);
+  o.z = pack2<BF16>(acc[4] * inv, acc[5] * inv);
+  o.w = pack2<BF16>(acc[6] * inv, acc[7] * inv);
+  *reinterpret_cast<uint4*>(ctx + static_cast<size_t>(tok0 + (row & 63)) * hidden + head * 64 + col) = o;
 }
 
 }  // namespace
@@ -690,10 +697,10 @@ rt_status launch_sparse_attention(void* ctx, const void* q, const void* k, const
     RT_REQUIRE(split.groups_dev && split.part_o && split.part_ml, RT_ERR_INVALID,
                "sparse_attention: split lists without partial-result scratch");
     if (dtype == RT_BF16)
-      RT_CHECK_CUDA(launch_kernel(merge_partials_kernel<true>, dim3(split.n_groups), dim3(128), 0, st, (uint16_t*)ctx,
+      RT_CHECK_CUDA(launch_kernel(merge_partials_kernel<true>, dim3(split.n_groups, kMergeCtas), dim3(8 * kMergeRows), 0, st, (uint16_t*)ctx,
                                   split.groups_dev, (const float*)split.part_o, (const float*)split.part_ml, hidden));
     else
-      RT_CHECK_CUDA(launch_kernel(merge_partials_kernel<false>, dim3(split.n_groups), dim3(128), 0, st, (uint16_t*)ctx,
+      RT_CHECK_CUDA(launch_kernel(merge_partials_kernel<false>, dim3(split.n_groups, kMergeCtas), dim3(8 * kMergeRows), 0, st, (uint16_t*)ctx,
                                   split.groups_dev, (const float*)split.part_o, (const float*)split.part_ml, hidden));
     count_launch();
     RT_CHECK_CUDA(cudaGetLastError());
