@@ -59,6 +59,22 @@ struct Vec8<__nv_bfloat16> {
   }
 };
 
+// four 16-bit values at once (64 bits)
+template <typename T>
+__device__ __forceinline__ void unpack4(const T* p, float* f) {
+  const uint2 w = *reinterpret_cast<const uint2*>(p);
+  float t[8];
+  Vec8<T>::unpack(make_uint4(w.x, w.y, 0u, 0u), t);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) f[i] = t[i];
+}
+template <typename T>
+__device__ __forceinline__ void pack4(const float* f, T* p) {
+  const float t[8] = {f[0], f[1], f[2], f[3], 0.f, 0.f, 0.f, 0.f};
+  const uint4 w = Vec8<T>::pack(t);
+  *reinterpret_cast<uint2*>(p) = make_uint2(w.x, w.y);
+}
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -158,6 +174,60 @@ layernorm_kernel(T* __restrict__ out, const T* __restrict__ x, const T* __restri
       }
     }
   }
+}
+
+// ---------------------------------------------------------------------------
+// The same over a projection given as `splits` fp32 parts [splits][rows][hidden] (split-K GEMM): sums the
+// parts, adds bias and residual, normalises.  One CTA per row, four columns per thread: used for batches of
+// few rows, where the latency of the part loads bounds it (all parts of a row are in flight together) and one
+// warp per row would leave most SMs without work.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ float block_sum(float v, float* s_warp) {
+  v = warp_sum(v);
+  const int warps = blockDim.x >> 5;
+  if ((threadIdx.x & 31) == 0) s_warp[threadIdx.x >> 5] = v;
+  __syncthreads();
+  float t = 0.f;
+  for (int i = 0; i < warps; ++i) t += s_warp[i];
+  return t;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(1024) layernorm_parts_kernel(T* __restrict__ out, const float* __restrict__ parts,
+                                                               const T* __restrict__ bias,
+                                                               const T* __restrict__ residual,
+                                                               const T* __restrict__ gamma, const T* __restrict__ beta,
+                                                               int rows, int hidden, int splits, float eps) {
+  __shared__ float s_sum[32], s_sq[32];
+  RT_PDL_LAUNCH_DEPENDENTS();
+  const int col = threadIdx.x * 4;
+  const size_t at = static_cast<size_t>(blockIdx.x) * hidden + col;
+  const float inv_h = 1.0f / static_cast<float>(hidden);
+  float bb[4], gg[4], be[4], rr[4], v[4] = {0.f, 0.f, 0.f, 0.f};
+  unpack4(bias + col, bb);
+  unpack4(gamma + col, gg);
+  unpack4(beta + col, be);
+  RT_PDL_WAIT();
+  unpack4(residual + at, rr);
+  const size_t stride = static_cast<size_t>(rows) * hidden;
+#pragma unroll 4
+  for (int s = 0; s < splits; ++s) {
+    const float4 p = *reinterpret_cast<const float4*>(parts + s * stride + at);
+    v[0] += p.x;
+    v[1] += p.y;
+    v[2] += p.z;
+    v[3] += p.w;
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) v[k] += bb[k] + rr[k];
+  const float mean = block_sum(v[0] + v[1] + v[2] + v[3], s_sum) * inv_h;
+  float sq = 0.f;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) sq += (v[k] - mean) * (v[k] - mean);
+  const float rstd = rsqrtf(block_sum(sq, s_sq) * inv_h + eps);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) v[k] = (v[k] - mean) * rstd * gg[k] + be[k];
+  pack4(v, out + at);
 }
 
 // ---------------------------------------------------------------------------
@@ -372,6 +442,23 @@ static rt_status layernorm_launch(void* out, const void* x, const void* bias, co
       return fail(RT_ERR_UNSUPPORTED, "layernorm: hidden=%d not supported (<=1024, 1536 or 2048)", hidden);
   }
 #undef RT_LN_CASE
+  count_launch();
+  RT_CHECK_CUDA(cudaGetLastError());
+  return RT_OK;
+}
+
+// out = LayerNorm(sum of the parts + bias + residual) * gamma + beta; hidden % 128 == 0, hidden <= 4096
+rt_status layernorm_parts(void* out, const float* parts, int splits, const void* bias, const void* residual,
+                          const void* gamma, const void* beta, int rows, int hidden, float eps, int dtype,
+                          cudaStream_t st) {
+  if (dtype == RT_BF16)
+    RT_CHECK_CUDA(launch_kernel(layernorm_parts_kernel<__nv_bfloat16>, dim3(rows), dim3(hidden / 4), 0, st,
+                                (__nv_bfloat16*)out, parts, (const __nv_bfloat16*)bias, (const __nv_bfloat16*)residual,
+                                (const __nv_bfloat16*)gamma, (const __nv_bfloat16*)beta, rows, hidden, splits, eps));
+  else
+    RT_CHECK_CUDA(launch_kernel(layernorm_parts_kernel<__half>, dim3(rows), dim3(hidden / 4), 0, st, (__half*)out, parts,
+                                (const __half*)bias, (const __half*)residual, (const __half*)gamma, (const __half*)beta,
+                                rows, hidden, splits, eps));
   count_launch();
   RT_CHECK_CUDA(cudaGetLastError());
   return RT_OK;

@@ -73,14 +73,26 @@ struct QkvEpilogue {
   const int2* block_seq;  // per packed 64-token block: {first token of its sequence, sequence length}
   int heads;
   float q_scale;
+  int splits;  // kEpiPartial: parts of K
 };
 constexpr int kEpiQkv = 3;
+// Split-K form: C is fp32 [splits][M][N], part s holds the sum over its K range; no bias.  The reader of the
+// parts (layernorm_parts_kernel) adds them up.
+constexpr int kEpiPartial = 5;
 
 // One 32-column chunk of one accumulator row: r[] holds the fp32 accumulators.
-template <int BN, bool BF16, int EPI>
+template <bool BF16, int EPI>
 __device__ __forceinline__ void epilogue_chunk(const uint32_t* r, int c, int row, int n0, int M, int N,
                                                uint16_t* __restrict__ C, const uint16_t* __restrict__ bias,
                                                const QkvEpilogue& qkv) {
+  if constexpr (EPI == kEpiPartial) {
+    if (row < M) {
+      float* dst = reinterpret_cast<float*>(C) + static_cast<size_t>(row) * N + n0 + c * 32;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) st_global_v8(dst + 8 * q, r + 8 * q);
+    }
+    return;
+  }
   uint32_t o[16];
   if constexpr (EPI == RT_EPI_NONE) {
 #pragma unroll
@@ -147,23 +159,23 @@ __device__ __forceinline__ void epilogue_chunk(const uint32_t* r, int c, int row
   }
 }
 
-// Drains columns [32*c] for c = chunk0, chunk0+2, ... < BN/32 of one accumulator row, two
+// Drains columns [32*c] for c = chunk0, chunk0+2, ... < width/32 of one accumulator row, two
 // chunks per step so that the second TMEM load is in flight while the first chunk is processed.
 //   taddr: TMEM address of column 0 of this thread's lane quarter; row: global output row.
-template <int BN, bool BF16, int EPI>
-__device__ __forceinline__ void epilogue_row(uint32_t taddr, int row, int n0, int chunk0, int M, int N,
+template <bool BF16, int EPI>
+__device__ __forceinline__ void epilogue_row(int width, uint32_t taddr, int row, int n0, int chunk0, int M, int N,
                                              uint16_t* __restrict__ C, const uint16_t* __restrict__ bias,
                                              const QkvEpilogue& qkv) {
-  constexpr int kChunks = BN / 32;
+  const int chunks = width / 32;
 #pragma unroll 1
-  for (int c = chunk0; c < kChunks; c += 4) {
+  for (int c = chunk0; c < chunks; c += 4) {
     uint32_t r0[32], r1[32];
-    const bool two = c + 2 < kChunks;
+    const bool two = c + 2 < chunks;
     tmem_ld32(taddr + c * 32, r0);
     if (two) tmem_ld32(taddr + (c + 2) * 32, r1);
     tc_wait_ld();
-    epilogue_chunk<BN, BF16, EPI>(r0, c, row, n0, M, N, C, bias, qkv);
-    if (two) epilogue_chunk<BN, BF16, EPI>(r1, c + 2, row, n0, M, N, C, bias, qkv);
+    epilogue_chunk<BF16, EPI>(r0, c, row, n0, M, N, C, bias, qkv);
+    if (two) epilogue_chunk<BF16, EPI>(r1, c + 2, row, n0, M, N, C, bias, qkv);
   }
 }
 

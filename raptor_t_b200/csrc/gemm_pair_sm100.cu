@@ -41,7 +41,7 @@ constexpr int kSmemBytes = kStages * kStageBytes + 1024 + 256;
 template <bool BF16, int EPI>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
-                 uint16_t* __restrict__ C, const uint16_t* __restrict__ bias, int M, int N, int K, int* error_flag,
+                 const __grid_constant__ CUtensorMap map_wt, int main_tiles, int tail_w, uint16_t* __restrict__ C, const uint16_t* __restrict__ bias, int M, int N, int K, int* error_flag,
                  QkvEpilogue qkv) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -85,29 +85,54 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   const uint32_t tmem_base = *tmem_slot;
   AbortCtx ab{cta_abort, error_flag};
 
-  const int n_tiles_n = N / kTileN;
   const int n_tiles_m = (M + kTileM - 1) / kTileM;
-  const int n_tiles = n_tiles_m * n_tiles_n;
+  const int tail_n = N / tail_w;                      // tiles of tail_w columns per row block
+  const int tail0 = main_tiles ? main_tiles * (kTileN / tail_w) : 0;  // of these, covered by the main tiles
+  const int mn_tiles = main_tiles + n_tiles_m * tail_n - tail0;
+  const int splits = EPI == kEpiPartial ? qkv.splits : 1;
+  const int n_tiles = mn_tiles * splits;
   const int k_blocks = K / kBK;
+  struct Tile {
+    int m0, n0, width, kb0, kb1, part;
+  };
+  // tile t: 256 columns wide up to main_tiles, then tail_w; over K blocks [kb0, kb1) of part t / mn_tiles
+  auto tile_of = [&](int t) {
+    Tile r;
+    r.part = EPI == kEpiPartial ? t / mn_tiles : 0;
+    const int u = EPI == kEpiPartial ? t % mn_tiles : t;
+    const bool main = u < main_tiles;
+    const int per_row = main ? N / kTileN : tail_n;
+    const int i = main ? u : u - main_tiles + tail0;
+    r.width = main ? kTileN : tail_w;
+    r.m0 = (i / per_row) * kTileM;
+    r.n0 = (i % per_row) * r.width;
+    r.kb0 = EPI == kEpiPartial ? r.part * k_blocks / splits : 0;
+    r.kb1 = EPI == kEpiPartial ? (r.part + 1) * k_blocks / splits : k_blocks;
+    return r;
+  };
 
   if (warp == 0) {
     // ------------------------------------------------------------- TMA producer (both CTAs)
     if (lane == 0) {
       prefetch_tensormap(&map_a);
       prefetch_tensormap(&map_w);
+      prefetch_tensormap(&map_wt);
       uint32_t it = 0;
       bool ok = true;
       for (int t = pair; t < n_tiles && ok; t += n_pairs) {
-        const int m0 = (t / n_tiles_n) * kTileM + rank * 128;
-        const int n0 = (t % n_tiles_n) * kTileN + rank * 128;
-        for (int kb = 0; kb < k_blocks; ++kb, ++it) {
+        const Tile tl = tile_of(t);
+        const int m0 = tl.m0 + rank * 128;
+        const int n0 = tl.n0 + rank * (tl.width / 2);
+        const CUtensorMap* mw = t % mn_tiles < main_tiles ? &map_w : &map_wt;
+        const uint32_t bytes = 2 * (kABytes + (tl.width / 2) * kBK * 2);  // of both CTAs
+        for (int kb = tl.kb0; kb < tl.kb1; ++kb, ++it) {
           const int s = it % kStages;
           const uint32_t ph = (it / kStages) & 1;
           if (!mbar_wait(&empty[s], ph ^ 1, ab, 111)) { ok = false; break; }
           uint8_t* sa = smem + s * kStageBytes;
-          if (rank == 0) mbar_arrive_expect_tx(&full[s], 2 * kStageBytes);  // both CTAs' bytes
+          if (rank == 0) mbar_arrive_expect_tx(&full[s], bytes);
           tma_load_2d_pair(sa, &map_a, kb * kBK, m0, &full[s]);
-          tma_load_2d_pair(sa + kABytes, &map_w, kb * kBK, n0, &full[s]);
+          tma_load_2d_pair(sa + kABytes, mw, kb * kBK, n0, &full[s]);
         }
       }
     }
@@ -118,7 +143,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     // every descriptor is moved over from a per-thread register first, and that serial latency per
     // 64-wide K slice is of the order of the slice's 512 clocks of MMA work).
     if (rank == 0) {
-      constexpr uint32_t idesc = make_idesc_f16(kTileM, kTileN, BF16 ? 1 : 0, false);
       const bool leader = elect_one();
       const uint32_t smem_base = smem_u32(smem);
       uint32_t it = 0, tile_it = 0;
@@ -129,7 +153,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         if (!mbar_wait(&acc_empty[a], aph ^ 1, ab, 112)) { ok = false; break; }
         tc_fence_after_sync();
         const uint32_t d_tmem = tmem_base + a * kTileN;
-        for (int kb = 0; kb < k_blocks; ++kb, ++it) {
+        const Tile tl = tile_of(t);
+        const uint32_t idesc = make_idesc_f16(kTileM, tl.width, BF16 ? 1 : 0, false);
+        for (int kb = tl.kb0; kb < tl.kb1; ++kb, ++it) {
           const int s = it % kStages;
           const uint32_t ph = (it / kStages) & 1;
           if (!mbar_wait(&full[s], ph, ab, 113)) { ok = false; break; }
@@ -140,7 +166,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
           if (leader) {
 #pragma unroll
             for (int k = 0; k < kBK / 16; ++k)
-              mma_ss_pair(d_tmem, da + (k * 32 >> 4), db + (k * 32 >> 4), idesc, (kb | k) ? 1u : 0u);
+              mma_ss_pair(d_tmem, da + (k * 32 >> 4), db + (k * 32 >> 4), idesc, kb > tl.kb0 || k > 0 ? 1u : 0u);
             tc_commit_pair(&empty[s], 3);  // slot free in both CTAs
           }
           __syncwarp();
@@ -160,12 +186,13 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     for (int t = pair; t < n_tiles && ok; t += n_pairs, ++tile_it) {
       const int a = tile_it & 1;
       const uint32_t aph = (tile_it >> 1) & 1;
-      const int m0 = (t / n_tiles_n) * kTileM, n0 = (t % n_tiles_n) * kTileN;
+      const Tile tl = tile_of(t);
       if (!mbar_wait(&acc_full[a], aph, ab, 114)) { ok = false; break; }
       tc_fence_after_sync();
-      const int row = m0 + row_in_tile;
+      const int row = tl.m0 + row_in_tile;
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + a * kTileN;
-      epilogue_row<kTileN, BF16, EPI>(taddr, row, n0, chunk0, M, N, C, bias, qkv);
+      uint16_t* c_part = EPI == kEpiPartial ? C + 2 * static_cast<size_t>(tl.part) * M * N : C;  // fp32 parts
+      epilogue_row<BF16, EPI>(tl.width, taddr, row, tl.n0, chunk0, M, N, c_part, bias, qkv);
       tc_fence_before_sync();
       mbar_arrive_cluster(leader_acc_empty[a]);
     }
@@ -183,18 +210,20 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 
 template <bool BF16, int EPI>
 rt_status launch_pair(void* c, const void* a, const void* w, const void* bias, int M, int N, int K, cudaStream_t st,
-                      const QkvEpilogue& qkv) {
-  CUtensorMap ma, mw;
+                      const QkvEpilogue& qkv, int main_tiles, int tail_w) {
+  CUtensorMap ma, mw, mwt;
   RT_TRY(make_tensor_map_2d(&ma, a, M, K, K, 128, kBK, true));
   RT_TRY(make_tensor_map_2d(&mw, w, N, K, K, 128, kBK, true));
+  RT_TRY(make_tensor_map_2d(&mwt, w, N, K, K, tail_w / 2, kBK, true));
   auto kern = gemm_pair_kernel<BF16, EPI>;
   RT_TRY(ensure_kernel_smem(reinterpret_cast<const void*>(kern), kSmemBytes, false));
   int* err = device_error_word();
   RT_REQUIRE(err != nullptr, RT_ERR_CUDA, "gemm: cannot allocate the device error word");
   const int sms = gemm_sm_count();
-  const int tiles = ((M + kTileM - 1) / kTileM) * (N / kTileN);
+  const int mn = main_tiles + ((M + kTileM - 1) / kTileM) * (N / tail_w) - (main_tiles ? main_tiles * (kTileN / tail_w) : 0);
+  const int tiles = mn * (EPI == kEpiPartial ? qkv.splits : 1);
   const int pairs = std::min(tiles, sms / 2);
-  RT_CHECK_CUDA(launch_kernel(kern, dim3(2 * pairs), dim3(kThreads), kSmemBytes, st, ma, mw, (uint16_t*)c,
+  RT_CHECK_CUDA(launch_kernel(kern, dim3(2 * pairs), dim3(kThreads), kSmemBytes, st, ma, mw, mwt, main_tiles, tail_w, (uint16_t*)c,
                               (const uint16_t*)bias, M, N, K, err, qkv));
   count_launch();
   RT_CHECK_CUDA(cudaGetLastError());
@@ -205,23 +234,26 @@ rt_status launch_pair(void* c, const void* a, const void* w, const void* bias, i
 
 // Entry used by rt_gemm / rt_gemm_qkv when the shape suits 256 x 256 pair tiles.
 rt_status gemm_pair_dispatch(void* c, const void* a, const void* w, const void* bias, int M, int N, int K, int epi,
-                             bool bf16, cudaStream_t st, const gemm_detail::QkvEpilogue& qkv) {
+                             bool bf16, cudaStream_t st, const gemm_detail::QkvEpilogue& qkv, int main_tiles, int tail_w) {
   switch (epi) {
     case RT_EPI_NONE:
-      return bf16 ? launch_pair<true, RT_EPI_NONE>(c, a, w, bias, M, N, K, st, qkv)
-                  : launch_pair<false, RT_EPI_NONE>(c, a, w, bias, M, N, K, st, qkv);
+      return bf16 ? launch_pair<true, RT_EPI_NONE>(c, a, w, bias, M, N, K, st, qkv, main_tiles, tail_w)
+                  : launch_pair<false, RT_EPI_NONE>(c, a, w, bias, M, N, K, st, qkv, main_tiles, tail_w);
     case RT_EPI_BIAS:
-      return bf16 ? launch_pair<true, RT_EPI_BIAS>(c, a, w, bias, M, N, K, st, qkv)
-                  : launch_pair<false, RT_EPI_BIAS>(c, a, w, bias, M, N, K, st, qkv);
+      return bf16 ? launch_pair<true, RT_EPI_BIAS>(c, a, w, bias, M, N, K, st, qkv, main_tiles, tail_w)
+                  : launch_pair<false, RT_EPI_BIAS>(c, a, w, bias, M, N, K, st, qkv, main_tiles, tail_w);
     case RT_EPI_BIAS_GELU:
-      return bf16 ? launch_pair<true, RT_EPI_BIAS_GELU>(c, a, w, bias, M, N, K, st, qkv)
-                  : launch_pair<false, RT_EPI_BIAS_GELU>(c, a, w, bias, M, N, K, st, qkv);
+      return bf16 ? launch_pair<true, RT_EPI_BIAS_GELU>(c, a, w, bias, M, N, K, st, qkv, main_tiles, tail_w)
+                  : launch_pair<false, RT_EPI_BIAS_GELU>(c, a, w, bias, M, N, K, st, qkv, main_tiles, tail_w);
     case RT_EPI_BIAS_RESIDUAL:
-      return bf16 ? launch_pair<true, RT_EPI_BIAS_RESIDUAL>(c, a, w, bias, M, N, K, st, qkv)
-                  : launch_pair<false, RT_EPI_BIAS_RESIDUAL>(c, a, w, bias, M, N, K, st, qkv);
+      return bf16 ? launch_pair<true, RT_EPI_BIAS_RESIDUAL>(c, a, w, bias, M, N, K, st, qkv, main_tiles, tail_w)
+                  : launch_pair<false, RT_EPI_BIAS_RESIDUAL>(c, a, w, bias, M, N, K, st, qkv, main_tiles, tail_w);
+    case gemm_detail::kEpiPartial:
+      return bf16 ? launch_pair<true, gemm_detail::kEpiPartial>(c, a, w, bias, M, N, K, st, qkv, main_tiles, tail_w)
+                  : launch_pair<false, gemm_detail::kEpiPartial>(c, a, w, bias, M, N, K, st, qkv, main_tiles, tail_w);
     case gemm_detail::kEpiQkv:
-      return bf16 ? launch_pair<true, gemm_detail::kEpiQkv>(c, a, w, bias, M, N, K, st, qkv)
-                  : launch_pair<false, gemm_detail::kEpiQkv>(c, a, w, bias, M, N, K, st, qkv);
+      return bf16 ? launch_pair<true, gemm_detail::kEpiQkv>(c, a, w, bias, M, N, K, st, qkv, main_tiles, tail_w)
+                  : launch_pair<false, gemm_detail::kEpiQkv>(c, a, w, bias, M, N, K, st, qkv, main_tiles, tail_w);
   }
   return fail(RT_ERR_INVALID, "gemm: unknown epilogue %d", epi);
 }

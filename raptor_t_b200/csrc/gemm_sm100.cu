@@ -17,6 +17,7 @@
 #include "common.h"
 #include "device_error.h"
 #include "gemm_epilogue.cuh"
+#include "gemm_plan.h"
 #include "launch.h"
 #include "launch_count.h"
 #include "sm100_ptx.cuh"
@@ -48,6 +49,22 @@ constexpr int kBM = 128;
 constexpr int kBK = 64;
 constexpr int kGemmThreads = 320;      // warp 0 TMA, warp 1 MMA, warps 2-9 epilogue
 constexpr int kEpilogueThreads = 256;  // two warps per TMEM lane quarter, alternating 32-column chunks
+
+// Costs of the tile choice (plan_gemm), microseconds on a B200 with weights and activations in L2, fitted to
+// M = 128 ... 20480 rows of the projections of 768- and 1024-wide models: per launch, per 64-wide K block of a
+// tile, per tile.  A 256-column pair tile does the most work per byte it loads and wins once its waves are full;
+// below that, narrower tiles on more SMs are faster (768 columns, K = 3072, 4096 rows: 48 pair tiles of 256
+// columns 19.9 us, 64 of 192 15.9 us, 192 single-CTA tiles of 128 25.1 us).
+struct TileCost {
+  int width;
+  double launch, k_block, tile;
+  double at(int waves, int k_blocks) const { return launch + waves * (k_blocks * k_block + tile); }
+};
+constexpr TileCost kSingleTiles[3] = {{64, 2.3, 0.2, 0.45}, {128, 2.6, 0.235, 0.6}, {256, 3.2, 0.285, 2.1}};
+constexpr TileCost kPairTiles[3] = {{128, 3.6, 0.2, 0.6}, {192, 3.6, 0.24, 1.3}, {256, 3.8, 0.29, 1.55}};
+// the last, partial wave of 256-column pair tiles cut into narrower ones
+constexpr TileCost kTailTiles[2] = {{64, 0, 0.15, 0.5}, {128, 0, 0.2, 0.6}};
+constexpr double kPartBytesPerUs = 6e6;  // fp32 parts, written and read through L2
 
 template <int BN>
 struct GemmCfg {
@@ -104,8 +121,20 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
 
   const int n_tiles_n = N / BN;
   const int n_tiles_m = (M + kBM - 1) / kBM;
-  const int n_tiles = n_tiles_m * n_tiles_n;
+  const int mn_tiles = n_tiles_m * n_tiles_n;
+  const int splits = EPI == kEpiPartial ? qkv.splits : 1;
+  const int n_tiles = mn_tiles * splits;
   const int k_blocks = K / kBK;
+  // tile t: output tile t % mn_tiles over K blocks [kb0, kb1) of part t / mn_tiles
+  auto tile_of = [&](int t, int& m0, int& n0, int& kb0, int& kb1, int& part) {
+    part = EPI == kEpiPartial ? t / mn_tiles : 0;
+    const int u = EPI == kEpiPartial ? t % mn_tiles : t;
+    m0 = (u / n_tiles_n) * kBM;
+    n0 = (u % n_tiles_n) * BN;
+    kb0 = EPI == kEpiPartial ? part * k_blocks / splits : 0;
+    kb1 = EPI == kEpiPartial ? (part + 1) * k_blocks / splits : k_blocks;
+  };
+  int m0, n0, kb0, kb1, part;
 
   if (warp == 0) {
     // ------------------------------------------------------------- TMA producer
@@ -115,8 +144,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
       uint32_t it = 0;
       bool ok = true;
       for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
-        const int m0 = (t / n_tiles_n) * kBM, n0 = (t % n_tiles_n) * BN;
-        for (int kb = 0; kb < k_blocks; ++kb, ++it) {
+        tile_of(t, m0, n0, kb0, kb1, part);
+        for (int kb = kb0; kb < kb1; ++kb, ++it) {
           const int s = it % Cfg::kStages;
           const uint32_t ph = (it / Cfg::kStages) & 1;
           if (!mbar_wait(&empty[s], ph ^ 1, ab, 101)) { ok = false; break; }
@@ -145,7 +174,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         if (!mbar_wait(&acc_empty[a], aph ^ 1, ab, 102)) { ok = false; break; }
         tc_fence_after_sync();
         const uint32_t d_tmem = tmem_base + a * BN;
-        for (int kb = 0; kb < k_blocks; ++kb, ++it) {
+        tile_of(t, m0, n0, kb0, kb1, part);
+        for (int kb = kb0; kb < kb1; ++kb, ++it) {
           const int s = it % Cfg::kStages;
           const uint32_t ph = (it / Cfg::kStages) & 1;
           if (!mbar_wait(&full[s], ph, ab, 103)) { ok = false; break; }
@@ -156,7 +186,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
           if (elected) {
 #pragma unroll
             for (int k = 0; k < kBK / 16; ++k)
-              mma_ss(d_tmem, da + (k * 32 >> 4), db + (k * 32 >> 4), idesc, (kb | k) ? 1u : 0u);
+              mma_ss(d_tmem, da + (k * 32 >> 4), db + (k * 32 >> 4), idesc, kb > kb0 || k > 0 ? 1u : 0u);
             tc_commit(&empty[s]);
           }
           __syncwarp();
@@ -175,12 +205,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x, ++tile_it) {
       const int a = tile_it & 1;
       const uint32_t aph = (tile_it >> 1) & 1;
-      const int m0 = (t / n_tiles_n) * kBM, n0 = (t % n_tiles_n) * BN;
+      tile_of(t, m0, n0, kb0, kb1, part);
       if (!mbar_wait(&acc_full[a], aph, ab, 104)) { ok = false; break; }
       tc_fence_after_sync();
       const int row = m0 + row_in_tile;
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + a * BN;
-      epilogue_row<BN, BF16, EPI>(taddr, row, n0, chunk0, M, N, C, bias, qkv);
+      uint16_t* c_part = EPI == kEpiPartial ? C + 2 * static_cast<size_t>(part) * M * N : C;  // fp32 parts
+      epilogue_row<BF16, EPI>(BN, taddr, row, n0, chunk0, M, N, c_part, bias, qkv);
       tc_fence_before_sync();
       mbar_arrive(&acc_empty[a]);
     }
@@ -205,7 +236,7 @@ rt_status launch(void* c, const void* a, const void* w, const void* bias, int M,
   RT_TRY(ensure_kernel_smem(reinterpret_cast<const void*>(kern), Cfg::kSmemBytes, false));
   int* err = device_error_word();
   RT_REQUIRE(err != nullptr, RT_ERR_CUDA, "gemm: cannot allocate the device error word");
-  const int tiles = ((M + kBM - 1) / kBM) * (N / BN);
+  const int tiles = ((M + kBM - 1) / kBM) * (N / BN) * (EPI == kEpiPartial ? qkv.splits : 1);
   const int grid = std::min(tiles, gemm_sm_count());
   RT_CHECK_CUDA(launch_kernel(kern, dim3(grid), dim3(kGemmThreads), Cfg::kSmemBytes, st, ma, mw, (uint16_t*)c,
                               (const uint16_t*)bias, M, N, K, err, qkv));
@@ -216,12 +247,14 @@ rt_status launch(void* c, const void* a, const void* w, const void* bias, int M,
 
 template <int BN, bool BF16>
 rt_status launch_epi(void* c, const void* a, const void* w, const void* bias, int M, int N, int K, int epi,
-                     cudaStream_t st, const QkvEpilogue& qkv = QkvEpilogue{}) {
+                     cudaStream_t st, const QkvEpilogue& qkv) {
   switch (epi) {
     case RT_EPI_NONE: return launch<BN, BF16, RT_EPI_NONE>(c, a, w, bias, M, N, K, st);
     case RT_EPI_BIAS: return launch<BN, BF16, RT_EPI_BIAS>(c, a, w, bias, M, N, K, st);
     case RT_EPI_BIAS_GELU: return launch<BN, BF16, RT_EPI_BIAS_GELU>(c, a, w, bias, M, N, K, st);
     case RT_EPI_BIAS_RESIDUAL: return launch<BN, BF16, RT_EPI_BIAS_RESIDUAL>(c, a, w, bias, M, N, K, st, qkv);
+    case kEpiQkv: return launch<BN, BF16, kEpiQkv>(c, a, w, bias, M, N, K, st, qkv);
+    case kEpiPartial: return launch<BN, BF16, kEpiPartial>(c, a, w, bias, M, N, K, st, qkv);
   }
   return fail(RT_ERR_INVALID, "gemm: unknown epilogue %d", epi);
 }
@@ -229,11 +262,44 @@ rt_status launch_epi(void* c, const void* a, const void* w, const void* bias, in
 }  // namespace
 
 rt_status gemm_pair_dispatch(void* c, const void* a, const void* w, const void* bias, int M, int N, int K, int epi,
-                             bool bf16, cudaStream_t st, const gemm_detail::QkvEpilogue& qkv);
+                             bool bf16, cudaStream_t st, const gemm_detail::QkvEpilogue& qkv, int main_tiles, int tail_w);
 
-// 256 x 256 CTA-pair tiles pay off when there are enough of them to fill the SM pairs.
-static bool use_pair_tiles(int M, int N) {
-  return N % 256 == 0 && ((M + 255) / 256) * (N / 256) >= gemm_sm_count() / 2;
+GemmPlan plan_gemm(int M, int N, int K, int max_splits, bool to_parts) {
+  const int sms = gemm_sm_count(), pairs = sms / 2;
+  const int mt = (M + kBM - 1) / kBM, pair_mt = (M + 2 * kBM - 1) / (2 * kBM);
+  GemmPlan best;
+  best.cost = 1e30;
+  auto waves = [](int tiles, int units) { return (tiles + units - 1) / units; };
+  for (int s = 1; s <= max_splits; ++s) {
+    const int kbs = (K / kBK + s - 1) / s;
+    const double parts = to_parts ? 8.0 * s * M * N / kPartBytesPerUs : 0.0;
+    auto consider = [&](double cost, bool pair, int main_tiles, int width) {
+      if (cost + parts < best.cost) best = GemmPlan{pair, main_tiles, width, s, cost + parts};
+    };
+    for (const TileCost& c : kSingleTiles)
+      if (N % c.width == 0) consider(c.at(waves(mt * (N / c.width) * s, sms), kbs), false, 0, c.width);
+    for (const TileCost& c : kPairTiles)
+      if (N % c.width == 0) consider(c.at(waves(pair_mt * (N / c.width) * s, pairs), kbs), true, 0, c.width);
+    // whole waves of 256-column pair tiles, the rest in narrower ones (5003 rows, 3072 columns, K = 768:
+    // 222 + 18 tiles of 256 columns 22.7 us, 222 and 72 of 64 columns 21.2 us)
+    const int tiles = pair_mt * (N / 256), full = tiles / pairs, rest = tiles % pairs;
+    if (to_parts || N % 256 != 0 || full == 0 || rest == 0) continue;
+    for (const TileCost& c : kTailTiles)
+      consider(kPairTiles[2].at(full, kbs) + c.at(waves(rest * (256 / c.width), pairs), kbs), true, full * pairs, c.width);
+  }
+  return best;
+}
+
+rt_status run_gemm(void* c, const void* a, const void* w, const void* bias, int M, int N, int K, int epi, int dtype,
+                   cudaStream_t st, const gemm_detail::QkvEpilogue& extra, const GemmPlan& plan) {
+  const bool bf = dtype == RT_BF16;
+  if (plan.pair) return gemm_pair_dispatch(c, a, w, bias, M, N, K, epi, bf, st, extra, plan.main_tiles, plan.width);
+  if (plan.width == 256) return bf ? launch_epi<256, true>(c, a, w, bias, M, N, K, epi, st, extra)
+                                   : launch_epi<256, false>(c, a, w, bias, M, N, K, epi, st, extra);
+  if (plan.width == 128) return bf ? launch_epi<128, true>(c, a, w, bias, M, N, K, epi, st, extra)
+                                   : launch_epi<128, false>(c, a, w, bias, M, N, K, epi, st, extra);
+  return bf ? launch_epi<64, true>(c, a, w, bias, M, N, K, epi, st, extra)
+            : launch_epi<64, false>(c, a, w, bias, M, N, K, epi, st, extra);
 }
 
 }  // namespace rt
@@ -251,22 +317,7 @@ static rt_status gemm_entry(void* c, const void* a, const void* w, const void* b
              RT_ERR_INVALID, "gemm: A, W and bias must be 16-byte aligned, C 32-byte aligned");
   RT_REQUIRE(dtype == RT_F16 || dtype == RT_BF16, RT_ERR_INVALID, "gemm: unknown dtype %d", dtype);
   if (M == 0) return RT_OK;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (use_pair_tiles(M, N))
-    return gemm_pair_dispatch(c, a, w, bias, M, N, K, epilogue, dtype == RT_BF16, st, extra);
-  // largest tile width that divides N and still gives every SM a tile; else the narrowest
-  const int sms = gemm_sm_count();
-  const int mt = (M + kBM - 1) / kBM;
-  int bn = 64;
-  if (N % 256 == 0 && mt * (N / 256) >= sms) bn = 256;
-  else if (N % 128 == 0 && mt * (N / 128) >= sms) bn = 128;
-  const bool bf = dtype == RT_BF16;
-  if (bn == 256) return bf ? launch_epi<256, true>(c, a, w, bias, M, N, K, epilogue, st, extra)
-                           : launch_epi<256, false>(c, a, w, bias, M, N, K, epilogue, st, extra);
-  if (bn == 128) return bf ? launch_epi<128, true>(c, a, w, bias, M, N, K, epilogue, st, extra)
-                           : launch_epi<128, false>(c, a, w, bias, M, N, K, epilogue, st, extra);
-  return bf ? launch_epi<64, true>(c, a, w, bias, M, N, K, epilogue, st, extra)
-            : launch_epi<64, false>(c, a, w, bias, M, N, K, epilogue, st, extra);
+  return run_gemm(c, a, w, bias, M, N, K, epilogue, dtype, static_cast<cudaStream_t>(stream), extra, plan_gemm(M, N, K, 1, false));
 }
 
 extern "C" rt_status rt_gemm(void* c, const void* a, const void* w, const void* bias, int M, int N, int K, int epilogue,
@@ -300,18 +351,7 @@ extern "C" rt_status rt_gemm_qkv(void* q, void* k, void* v, const void* a, const
   if (M == 0) return RT_OK;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   QkvEpilogue e{nullptr, (uint16_t*)q, (uint16_t*)k, (uint16_t*)v, reinterpret_cast<const int2*>(block_seq_dev), heads,
-                q_scale};
-  if (use_pair_tiles(M, N)) return gemm_pair_dispatch(nullptr, a, w, bias, M, N, K, kEpiQkv, dtype == RT_BF16, st, e);
-  const int mt = (M + kBM - 1) / kBM;
-  // tile width must divide 3*heads*64 and keep a 32-column chunk inside one head: 64, 128 and 256 all do
-  const int sms = gemm_sm_count();
-  const bool wide = N % 256 == 0 && mt * (N / 256) >= sms;
-  const bool mid = N % 128 == 0 && mt * (N / 128) >= sms;
-  const bool bf = dtype == RT_BF16;
-  if (wide) return bf ? launch<256, true, kEpiQkv>(nullptr, a, w, bias, M, N, K, st, e)
-                      : launch<256, false, kEpiQkv>(nullptr, a, w, bias, M, N, K, st, e);
-  if (mid) return bf ? launch<128, true, kEpiQkv>(nullptr, a, w, bias, M, N, K, st, e)
-                     : launch<128, false, kEpiQkv>(nullptr, a, w, bias, M, N, K, st, e);
-  return bf ? launch<64, true, kEpiQkv>(nullptr, a, w, bias, M, N, K, st, e)
-            : launch<64, false, kEpiQkv>(nullptr, a, w, bias, M, N, K, st, e);
+                q_scale, 1};
+  // every tile width keeps a 32-column chunk inside one head
+  return run_gemm(nullptr, a, w, bias, M, N, K, kEpiQkv, dtype, st, e, plan_gemm(M, N, K, 1, false));
 }
