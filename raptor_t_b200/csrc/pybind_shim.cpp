@@ -167,6 +167,23 @@ struct LayerRegistry {
   std::vector<BertAttention*> layers;
   torch::Tensor block_seq;  // per packed 64-token block {first token of its sequence, length}: the fused QKV epilogue's map
   torch::Tensor seq_prefix; // int32 [B+1] block offsets of the sequences (device): the pooler's "first token" map
+  std::optional<c10::cuda::CUDAStream> upload_stream;  // both tensors belong to it
+  cudaEvent_t upload_done = nullptr;
+
+  void uploaded_on(const c10::cuda::CUDAStream& s) {
+    if (!upload_done) cudaEventCreateWithFlags(&upload_done, cudaEventDisableTiming);
+    cudaEventRecord(upload_done, s.stream());
+    upload_stream = s;
+  }
+  // Before the current stream reads them: a stream other than the uploading one waits for the copies and keeps
+  // the tensors' memory from being reused under its kernels.
+  void use_on_current_stream() {
+    const auto s = at::cuda::getCurrentCUDAStream();
+    if (!upload_stream || s == *upload_stream) return;
+    cudaStreamWaitEvent(s.stream(), upload_done, 0);
+    block_seq.record_stream(s);
+    seq_prefix.record_stream(s);
+  }
   static LayerRegistry& get() {
     static LayerRegistry r;
     return r;
@@ -275,6 +292,7 @@ class BertAttention {
     torch::Tensor dense = ts->get("dense_out", hidden_, st_dtype);
     void* st = stream_of_current();
     auto& reg = LayerRegistry::get();
+    reg.use_on_current_stream();
     if (kernel_fusion && reg.block_seq.defined() && info.find("add_bias_and_transpose_kernel") == info.end()) {
       check(rt_gemm_qkv(q.data_ptr(), k.data_ptr(), v.data_ptr(), input_tensor.data_ptr(), qkv_w_.data_ptr(),
                         qkv_b_.data_ptr(), reg.block_seq.data_ptr<int32_t>(), T, heads_, hidden_, 0.125f, dtype_, st));
@@ -305,6 +323,9 @@ class BertAttention {
     auto pre = info.find("pre_process");
     if (pre != info.end())
       pre->second += std::chrono::duration<float>(std::chrono::steady_clock::now() - t0).count();
+    if (plan_used_ && plan_stream_ != st) plan_shared_ = true;
+    plan_used_ = true;
+    plan_stream_ = st;
     timed(info, "attention", [&] {
       check(rt_sparse_attention(ctx.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), plan_, 1.0f, dtype_, st));
     });
@@ -324,10 +345,13 @@ class BertAttention {
       if (r.plan) rt_attn_plan_destroy(r.plan);
     }
     if (plan_) {
-      cudaDeviceSynchronize();  // the previous batch's attention kernel may still read it
-      rt_attn_plan_destroy(plan_);
+      // the previous batch's attention kernel may still read it: its memory is free again behind the stream that
+      // ran it; a plan that several streams used waits for the device
+      if (plan_used_ && !plan_shared_) rt_attn_plan_destroy_on(plan_, plan_stream_);
+      else rt_attn_plan_destroy(plan_);
       plan_ = nullptr;
     }
+    plan_used_ = plan_shared_ = false;
   }
 
   int heads_, hidden_ = 0, layer_idx_, dtype_ = RT_F16, device_ = 0;
@@ -336,6 +360,8 @@ class BertAttention {
   std::future<PlanResult> pending_;
   std::vector<int32_t> sync_lens_;
   rt_attn_plan* plan_ = nullptr;
+  bool plan_used_ = false, plan_shared_ = false;  // the current plan has been launched / from more than one stream
+  void* plan_stream_ = nullptr;
 };
 
 class MetaData {
@@ -363,9 +389,14 @@ class MetaData {
     }
     auto& reg = LayerRegistry::get();
     std::lock_guard<std::mutex> lk(reg.mu);
-    reg.block_seq = torch::from_blob(bs.data(), {static_cast<int64_t>(bs.size())}, torch::kInt32).clone().to(torch::kCUDA);
-    reg.seq_prefix = torch::from_blob(seq_len_info.data(), {static_cast<int64_t>(seq_len_info.size())}, torch::kInt32)
-                         .clone().to(torch::kCUDA);
+    // from pinned memory, so that the copies do not wait for the previous batch's kernels
+    auto upload = [](std::vector<int32_t>& v) {
+      return torch::from_blob(v.data(), {static_cast<int64_t>(v.size())}, torch::kInt32).pin_memory()
+          .to(torch::kCUDA, /*non_blocking=*/true);
+    };
+    reg.block_seq = upload(bs);
+    reg.seq_prefix = upload(seq_len_info);
+    reg.uploaded_on(at::cuda::getCurrentCUDAStream());
     for (BertAttention* l : reg.layers)
       if (l) l->kick(lens, device);
   }
@@ -460,6 +491,7 @@ class BertPooler {
     require_cuda(output, "output");
     auto& reg = LayerRegistry::get();
     if (!reg.seq_prefix.defined()) throw std::runtime_error("raptor_t: BertPooler called before MetaData.update_meta_data");
+    reg.use_on_current_stream();
     if (output.scalar_type() != torch::kFloat32) throw std::runtime_error("raptor_t: BertPooler writes a float32 output");
     check(rt_pooler(output.data_ptr<float>(), input_tensor.data_ptr(), reg.seq_prefix.data_ptr<int32_t>(),
                     static_cast<int>(reg.seq_prefix.numel()) - 1, w_.data_ptr(), b_.data_ptr(), hidden_, dtype_,
