@@ -134,7 +134,13 @@ struct rt_encoder {
   bool fuse_residual = false;  // measured slower on B200 (GEMM epilogue cost > LayerNorm saving); kept as an option
 
   // scratch ("TensorSet")
-  std::map<std::string, DevBuf> scratch;
+  struct Region {
+    void* p = nullptr;
+    size_t bytes = 0;
+  };
+  DevBuf scratch_mem;  // one allocation for all of them
+  std::map<std::string, Region> scratch;
+  Region ln_parts;     // fp32 split-K parts (plan_parts)
   int capacity_tokens = 0;
 
   // batch state
@@ -373,22 +379,27 @@ rt_status wait_layer_table(rt_encoder* e, int layer, cudaStream_t st) {
 }
 
 // split-K parts of a projection that LayerNorm sums up (plan_parts)
-constexpr int kMaxLnSplits = 12;
+constexpr int kMaxLnSplits = 6;  // more is no faster (128 rows: 8.3 us with 6 parts, 8.5 with 8)
 constexpr size_t kLnPartsBytes = 32u << 20;
 
 rt_status ensure_scratch(rt_encoder* e, int tokens) {
   if (tokens <= e->capacity_tokens) return RT_OK;
   const size_t T = tokens, H = e->cfg.hidden, F = e->cfg.ffn;
   RT_CHECK_CUDA(cudaDeviceSynchronize());
-  // the unfused QKV result; free again by the time FFN down leaves its split-K parts there (plan_parts)
-  RT_TRY(e->scratch["tmp_qkv_out1"].ensure(std::max(T * 3 * H * 2, std::min(T * H * 4 * kMaxLnSplits, kLnPartsBytes))));
-  RT_TRY(e->scratch["q_out"].ensure(T * H * 2));
-  RT_TRY(e->scratch["k_out"].ensure(T * H * 2));
-  RT_TRY(e->scratch["v_out"].ensure(T * H * 2));
-  RT_TRY(e->scratch["attention_out"].ensure(T * H * 2));
-  RT_TRY(e->scratch["dense_out"].ensure(T * H * 2));
-  RT_TRY(e->scratch["attention_output"].ensure(T * H * 2));
-  RT_TRY(e->scratch["intermediate"].ensure(T * F * 2));
+  const std::pair<const char*, size_t> names[] = {
+      {"tmp_qkv_out1", T * 3 * H * 2}, {"q_out", T * H * 2},        {"k_out", T * H * 2},
+      {"v_out", T * H * 2},            {"attention_out", T * H * 2}, {"dense_out", T * H * 2},
+      {"attention_output", T * H * 2}, {"intermediate", T * F * 2}};
+  const size_t parts = std::min(T * H * 4 * kMaxLnSplits, kLnPartsBytes);
+  size_t total = parts;
+  for (const auto& n : names) total += align256(n.second);
+  RT_TRY(e->scratch_mem.ensure(total));
+  uint8_t* at = static_cast<uint8_t*>(e->scratch_mem.p);
+  for (const auto& n : names) {
+    e->scratch[n.first] = {at, n.second};
+    at += align256(n.second);
+  }
+  e->ln_parts = {at, parts};
   e->capacity_tokens = tokens;
   return RT_OK;
 }
@@ -420,7 +431,7 @@ bool plan_parts(const rt_encoder* e, int K, GemmPlan& plan) {
 rt_status run_parts(rt_encoder* e, const GemmPlan& plan, const char* span, void* out, const void* a, const void* w,
                     const void* bias, const void* residual, const void* gamma, const void* beta, int K, cudaStream_t st) {
   const rt_config& c = e->cfg;
-  float* parts = static_cast<float*>(e->scratch["tmp_qkv_out1"].p);
+  float* parts = static_cast<float*>(e->ln_parts.p);
   gemm_detail::QkvEpilogue extra{};
   extra.splits = plan.splits;
   {
@@ -620,7 +631,7 @@ extern "C" rt_status rt_encoder_destroy(rt_encoder* e) {
   for (DevBuf* b : {&e->emb_word, &e->emb_pos, &e->emb_type, &e->emb_g, &e->emb_b, &e->ids_dev, &e->pos_dev, &e->part_o,
                     &e->part_ml})
     b->release();
-  for (auto& kv : e->scratch) kv.second.release();
+  e->scratch_mem.release();
   for (auto& slot : e->slots) {
     slot.meta_dev.release();
     slot.prefix_dev.release();
