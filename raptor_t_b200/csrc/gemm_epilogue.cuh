@@ -80,20 +80,10 @@ constexpr int kEpiQkv = 3;
 // parts (layernorm_parts_kernel) adds them up.
 constexpr int kEpiPartial = 5;
 
-// One 32-column chunk of one accumulator row: r[] holds the fp32 accumulators.
+// 32 columns, from `col` on, of one accumulator row: r[] holds the fp32 accumulators, o[] gets the 16-bit results.
 template <bool BF16, int EPI>
-__device__ __forceinline__ void epilogue_chunk(const uint32_t* r, int c, int row, int n0, int M, int N,
-                                               uint16_t* __restrict__ C, const uint16_t* __restrict__ bias,
-                                               const QkvEpilogue& qkv) {
-  if constexpr (EPI == kEpiPartial) {
-    if (row < M) {
-      float* dst = reinterpret_cast<float*>(C) + static_cast<size_t>(row) * N + n0 + c * 32;
-#pragma unroll
-      for (int q = 0; q < 4; ++q) st_global_v8(dst + 8 * q, r + 8 * q);
-    }
-    return;
-  }
-  uint32_t o[16];
+__device__ __forceinline__ void epilogue_values(const uint32_t* r, uint32_t* o, int col, int row, int M, int N,
+                                                const uint16_t* __restrict__ bias, const QkvEpilogue& qkv) {
   if constexpr (EPI == RT_EPI_NONE) {
 #pragma unroll
     for (int j = 0; j < 16; ++j) o[j] = pack2<BF16>(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
@@ -101,7 +91,7 @@ __device__ __forceinline__ void epilogue_chunk(const uint32_t* r, int c, int row
     uint32_t res[16];
     if constexpr (EPI == RT_EPI_BIAS_RESIDUAL) {
       if (row < M) {
-        const uint4* rp = reinterpret_cast<const uint4*>(qkv.residual + static_cast<size_t>(row) * N + n0 + c * 32);
+        const uint4* rp = reinterpret_cast<const uint4*>(qkv.residual + static_cast<size_t>(row) * N + col);
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
           const uint4 t = rp[q];
@@ -115,7 +105,7 @@ __device__ __forceinline__ void epilogue_chunk(const uint32_t* r, int c, int row
         for (int q = 0; q < 16; ++q) res[q] = 0u;
       }
     }
-    const uint4* bv = reinterpret_cast<const uint4*>(bias + n0 + c * 32);
+    const uint4* bv = reinterpret_cast<const uint4*>(bias + col);
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const uint4 b4 = __ldg(bv + q);
@@ -132,7 +122,7 @@ __device__ __forceinline__ void epilogue_chunk(const uint32_t* r, int c, int row
           x1 += rr.y;
         }
         if constexpr (EPI == kEpiQkv) {
-          if (n0 + c * 32 < qkv.heads * 64) {  // query part
+          if (col < qkv.heads * 64) {  // query part
             x0 *= qkv.q_scale;
             x1 *= qkv.q_scale;
           }
@@ -141,6 +131,23 @@ __device__ __forceinline__ void epilogue_chunk(const uint32_t* r, int c, int row
       }
     }
   }
+}
+
+// The same, stored by the thread itself.
+template <bool BF16, int EPI>
+__device__ __forceinline__ void epilogue_chunk(const uint32_t* r, int c, int row, int n0, int M, int N,
+                                               uint16_t* __restrict__ C, const uint16_t* __restrict__ bias,
+                                               const QkvEpilogue& qkv) {
+  if constexpr (EPI == kEpiPartial) {
+    if (row < M) {
+      float* dst = reinterpret_cast<float*>(C) + static_cast<size_t>(row) * N + n0 + c * 32;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) st_global_v8(dst + 8 * q, r + 8 * q);
+    }
+    return;
+  }
+  uint32_t o[16];
+  epilogue_values<BF16, EPI>(r, o, n0 + c * 32, row, M, N, bias, qkv);
   if (row < M) {
     uint16_t* dst;
     if constexpr (EPI == kEpiQkv) {
@@ -176,6 +183,55 @@ __device__ __forceinline__ void epilogue_row(int width, uint32_t taddr, int row,
     tc_wait_ld();
     epilogue_chunk<BF16, EPI>(r0, c, row, n0, M, N, C, bias, qkv);
     if (two) epilogue_chunk<BF16, EPI>(r1, c + 2, row, n0, M, N, C, bias, qkv);
+  }
+}
+
+// The tile through shared memory and TMA stores: warp `set` of a lane quarter takes the 64-column chunks set, set + 2,
+// ... of its 32 rows, writes them as 128-byte swizzled rows into its own 4 KB of `stage` and one lane stores
+// the box (rows past the last of the tensor are clipped).  Full 128-byte lines leave the SM, where a thread's own
+// 32-byte stores of a row each compete with the operand loads of the next tile.  20480 rows, K = 768: 3072 columns
+// with GELU 79.8 -> 74.2 us, QKV 60.1 -> 57.0; 4096 rows: 19.3 -> 17.6 and 14.7 -> 13.7.  drained() is called once
+// the accumulator has been read.
+template <bool BF16, int EPI, typename F>
+__device__ __forceinline__ void epilogue_tma(int width, uint32_t taddr, int row0, int lane, int n0, int set, int M,
+                                             int N, const uint16_t* __restrict__ bias, const QkvEpilogue& qkv,
+                                             uint8_t* stage, const CUtensorMap* map_c, const CUtensorMap* map_k,
+                                             const CUtensorMap* map_v, F&& drained) {
+  const int chunks = width / 64;
+  const int row = row0 + lane;
+  uint8_t* const line = stage + lane * 128;
+  const int swz = lane & 7;
+  if (set >= chunks) drained();
+#pragma unroll 1
+  for (int c = set; c < chunks; c += 2) {
+    uint32_t r[64], o[32];
+    tmem_ld32(taddr + c * 64, r);
+    tmem_ld32(taddr + c * 64 + 32, r + 32);
+    tc_wait_ld();
+    if (c + 2 >= chunks) drained();
+    const int col = n0 + c * 64;
+    epilogue_values<BF16, EPI>(r, o, col, row, M, N, bias, qkv);
+    epilogue_values<BF16, EPI>(r + 32, o + 16, col + 32, row, M, N, bias, qkv);
+    if (lane == 0) tma_store_wait_read<0>();  // the previous box has left the staging buffer
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      *reinterpret_cast<uint4*>(line + ((q ^ swz) << 4)) = make_uint4(o[4 * q], o[4 * q + 1], o[4 * q + 2], o[4 * q + 3]);
+    fence_proxy_async_smem();
+    __syncwarp();
+    if (lane == 0 && row0 < M) {
+      if constexpr (EPI == kEpiQkv) {
+        // a chunk is one head, and 32 rows stay inside one 64-token block: one box of the head-major matrix
+        const int hidden = qkv.heads * 64;
+        const int part = col / hidden;
+        const int2 bs = __ldg(qkv.block_seq + (row0 >> 6));
+        const int drow = bs.x * qkv.heads + ((col - part * hidden) >> 6) * bs.y + (row0 - bs.x);
+        tma_store_2d(part == 0 ? map_c : part == 1 ? map_k : map_v, stage, 0, drow);
+      } else {
+        tma_store_2d(map_c, stage, col, row0);
+      }
+      tma_store_commit();
+    }
   }
 }
 

@@ -36,16 +36,20 @@ constexpr int kStageBytes = kABytes + kBBytes;
 constexpr int kThreads = 320;           // warp 0 TMA, warp 1 MMA (leader only), warps 2-9 epilogue
 constexpr int kEpilogueThreads = 256;
 constexpr int kTmemCols = 512;          // two 256-column accumulators
-constexpr int kSmemBytes = kStages * kStageBytes + 1024 + 256;
+constexpr int kOutBytes = 32 * 64 * 2;   // one epilogue warp's output box
+constexpr int kSmemBytes = kStages * kStageBytes + 8 * kOutBytes + 1024 + 256;
+static_assert(kSmemBytes <= 227 * 1024, "shared memory of one CTA");
 
 template <bool BF16, int EPI>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
-                 const __grid_constant__ CUtensorMap map_wt, int main_tiles, int tail_w, uint16_t* __restrict__ C, const uint16_t* __restrict__ bias, int M, int N, int K, int* error_flag,
+                 const __grid_constant__ CUtensorMap map_wt, const __grid_constant__ CUtensorMap map_c,
+                 const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, int main_tiles, int tail_w, uint16_t* __restrict__ C, const uint16_t* __restrict__ bias, int M, int N, int K, int* error_flag,
                  QkvEpilogue qkv) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kStages * kStageBytes);
+  uint8_t* out_stage = smem + kStages * kStageBytes;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(out_stage + 8 * kOutBytes);
   uint64_t* full = bars;                  // leader's copy is the one in use
   uint64_t* empty = bars + kStages;       // each CTA waits on its own copy
   uint64_t* acc_full = bars + 2 * kStages;
@@ -179,7 +183,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     // ------------------------------------------------------------- epilogue warps 2..9 (both CTAs)
     const int quarter = warp & 3;
     const int chunk0 = (warp - 2) >> 2;
-    const int row_in_tile = rank * 128 + quarter * 32 + lane;
+    const int row_in_tile = rank * 128 + quarter * 32;
     const uint32_t leader_acc_empty[2] = {leader_smem_u32(&acc_empty[0]), leader_smem_u32(&acc_empty[1])};
     uint32_t tile_it = 0;
     bool ok = true;
@@ -189,13 +193,21 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       const Tile tl = tile_of(t);
       if (!mbar_wait(&acc_full[a], aph, ab, 114)) { ok = false; break; }
       tc_fence_after_sync();
-      const int row = tl.m0 + row_in_tile;
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + a * kTileN;
-      uint16_t* c_part = EPI == kEpiPartial ? C + 2 * static_cast<size_t>(tl.part) * M * N : C;  // fp32 parts
-      epilogue_row<BF16, EPI>(tl.width, taddr, row, tl.n0, chunk0, M, N, c_part, bias, qkv);
-      tc_fence_before_sync();
-      mbar_arrive_cluster(leader_acc_empty[a]);
+      auto drained = [&]() {
+        tc_fence_before_sync();
+        mbar_arrive_cluster(leader_acc_empty[a]);
+      };
+      if constexpr (EPI == kEpiPartial) {
+        uint16_t* c_part = C + 2 * static_cast<size_t>(tl.part) * M * N;  // fp32 parts
+        epilogue_row<BF16, EPI>(tl.width, taddr, tl.m0 + row_in_tile + lane, tl.n0, chunk0, M, N, c_part, bias, qkv);
+        drained();
+      } else {
+        epilogue_tma<BF16, EPI>(tl.width, taddr, tl.m0 + row_in_tile, lane, tl.n0, chunk0, M, N, bias, qkv,
+                                out_stage + (warp - 2) * kOutBytes, &map_c, &map_k, &map_v, drained);
+      }
     }
+    if (lane == 0) tma_store_wait<0>();  // the staging buffer is read and the output written before the CTA ends
   }
 
   tc_fence_before_sync();
@@ -211,10 +223,20 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 template <bool BF16, int EPI>
 rt_status launch_pair(void* c, const void* a, const void* w, const void* bias, int M, int N, int K, cudaStream_t st,
                       const QkvEpilogue& qkv, int main_tiles, int tail_w) {
-  CUtensorMap ma, mw, mwt;
+  CUtensorMap ma, mw, mwt, mc, mk, mv;
   RT_TRY(make_tensor_map_2d(&ma, a, M, K, K, 128, kBK, true));
   RT_TRY(make_tensor_map_2d(&mw, w, N, K, K, 128, kBK, true));
   RT_TRY(make_tensor_map_2d(&mwt, w, N, K, K, tail_w / 2, kBK, true));
+  if constexpr (EPI == kEpiQkv) {
+    const uint64_t rows = static_cast<uint64_t>(M) * qkv.heads;
+    RT_TRY(make_tensor_map_2d(&mc, qkv.q, rows, 64, 64, 32, 64, true));
+    RT_TRY(make_tensor_map_2d(&mk, qkv.k, rows, 64, 64, 32, 64, true));
+    RT_TRY(make_tensor_map_2d(&mv, qkv.v, rows, 64, 64, 32, 64, true));
+  } else {
+    if constexpr (EPI == kEpiPartial) mc = ma;  // fp32 parts are stored directly
+    else RT_TRY(make_tensor_map_2d(&mc, c, M, N, N, 32, 64, true));
+    mk = mv = mc;
+  }
   auto kern = gemm_pair_kernel<BF16, EPI>;
   RT_TRY(ensure_kernel_smem(reinterpret_cast<const void*>(kern), kSmemBytes, false));
   int* err = device_error_word();
@@ -223,7 +245,7 @@ rt_status launch_pair(void* c, const void* a, const void* w, const void* bias, i
   const int mn = main_tiles + ((M + kTileM - 1) / kTileM) * (N / tail_w) - (main_tiles ? main_tiles * (kTileN / tail_w) : 0);
   const int tiles = mn * (EPI == kEpiPartial ? qkv.splits : 1);
   const int pairs = std::min(tiles, sms / 2);
-  RT_CHECK_CUDA(launch_kernel(kern, dim3(2 * pairs), dim3(kThreads), kSmemBytes, st, ma, mw, mwt, main_tiles, tail_w, (uint16_t*)c,
+  RT_CHECK_CUDA(launch_kernel(kern, dim3(2 * pairs), dim3(kThreads), kSmemBytes, st, ma, mw, mwt, mc, mk, mv, main_tiles, tail_w, (uint16_t*)c,
                               (const uint16_t*)bias, M, N, K, err, qkv));
   count_launch();
   RT_CHECK_CUDA(cudaGetLastError());

@@ -61,7 +61,7 @@ struct TileCost {
   double at(int waves, int k_blocks) const { return launch + waves * (k_blocks * k_block + tile); }
 };
 constexpr TileCost kSingleTiles[3] = {{64, 2.3, 0.2, 0.45}, {128, 2.6, 0.235, 0.6}, {256, 3.2, 0.285, 2.1}};
-constexpr TileCost kPairTiles[3] = {{128, 3.6, 0.2, 0.6}, {192, 3.6, 0.24, 1.3}, {256, 3.8, 0.29, 1.55}};
+constexpr TileCost kPairTiles[3] = {{128, 3.6, 0.2, 0.5}, {192, 3.6, 0.24, 1.0}, {256, 3.8, 0.29, 1.2}};
 // the last, partial wave of 256-column pair tiles cut into narrower ones
 constexpr TileCost kTailTiles[2] = {{64, 0, 0.15, 0.5}, {128, 0, 0.2, 0.6}};
 constexpr double kPartBytesPerUs = 6e6;  // fp32 parts, written and read through L2
