@@ -405,9 +405,9 @@ rt_status ensure_scratch(rt_encoder* e, int tokens) {
 }
 
 // FFN down + LayerNorm for batches of few tokens: split-K GEMM into fp32 parts and a LayerNorm that sums them.
-// The cluster kernel takes 23 us for K = 3072 whether it has 128 or 4096 rows (one cluster of six CTAs per 256
-// rows walks all K blocks in sequence); cut along K until the chip is full, projection and LayerNorm take 8.3 us
-// for 128 rows, 11.7 for 1024, 16.9 for 2048 and 25.1 (against 24.9) for 4096.  Estimates in microseconds, as in
+// The cluster kernel walks all K blocks of a row block in sequence, however few row blocks there are (K = 3072:
+// 18.5 us for 128 rows, 19.8 for 2048, 21.7 for 4096); cut along K until the chip is full, projection and LayerNorm
+// take 8.3 us for 128 rows, 11.7 for 1024, 16.9 for 2048 and 25.1 for 4096.  Estimates in microseconds, as in
 // plan_gemm.  With K = 768 or 1024 the parts' traffic eats the gain (8.0 against 6.9 us for 128 rows): not used.
 bool plan_parts(const rt_encoder* e, int K, GemmPlan& plan) {
   const int M = e->tokens, N = e->cfg.hidden;
@@ -419,9 +419,9 @@ bool plan_parts(const rt_encoder* e, int K, GemmPlan& plan) {
   const double rows = static_cast<double>(M) * N;
   const double parts_cost = plan.cost + 2.5 + rows * 6 / 6e6;
   double other;
-  if (N == 768) {  // 22 clusters are resident; LayerNorm is part of their epilogue
-    const int waves = ((M + 255) / 256 + 21) / 22;
-    other = 3.5 + waves * (K / 64 * 0.38 + 0.9);
+  if (N == 768) {  // LayerNorm is part of the cluster kernel's epilogue; 36 clusters of 128 rows, 22 of 256 are resident
+    if (M <= 36 * 128) other = 8.5 + K / 64 * 0.21 + M * 0.00075;
+    else other = 3.5 + ((M + 255) / 256 + 21) / 22 * (K / 64 * 0.36 + 0.9);
   } else {
     other = plan_gemm(M, N, K, 1, false).cost + 1.9 + rows * 6 / 7.5e6;
   }
