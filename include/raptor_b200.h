@@ -298,11 +298,13 @@ rt_status rt_encoder_enable_timing(rt_encoder* enc, int on);
 rt_status rt_encoder_kernel_launches(rt_encoder* enc, int64_t* launches_out);
 /* options: "fuse_gelu" (1: bias+GELU in the FFN-up GEMM epilogue, 0: separate rt_bias_gelu kernel);
  * "fuse_qkv" (1: rt_gemm_qkv, 0: rt_gemm + rt_qkv_bias_transpose); "fuse_layernorm" (LayerNorm in the epilogue of
- * the hidden-wide projections, rt_gemm_bias_residual_layernorm: 0 never; 1 where it measured faster, i.e.
- * the FFN-down projection of a 768-wide model; 2 both projections of 768- and 1024-wide models);
+ * the hidden-wide projections of 768- and 1024-wide models, rt_gemm_bias_residual_layernorm: 0 never; 1 where it
+ * measured faster for the batch's token count, small batches take a split-K GEMM whose fp32 parts LayerNorm sums;
+ * 2 always);
  * "fuse_residual" (1: bias + residual added in the projection GEMM's epilogue, LayerNorm reads one tensor;
  * default 0: it costs one more 16-bit rounding and measured slower; ignored where fuse_layernorm applies).
- * fuse_gelu, fuse_qkv and fuse_layernorm default to 1. */
+ * fuse_gelu, fuse_qkv and fuse_layernorm default to 1.  rt_encoder_get_option also answers
+ * "layernorm_in_attention_output" and "layernorm_in_ffn_down": what the prepared batch does. */
 rt_status rt_encoder_set_option(rt_encoder* enc, const char* name, int value);
 rt_status rt_encoder_get_option(rt_encoder* enc, const char* name, int* value_out);
 /* work-list statistics of one layer of the prepared batch */

@@ -128,8 +128,8 @@ struct rt_encoder {
   bool fuse_gelu = true;
   bool fuse_qkv = true;
   // LayerNorm in the epilogue of the hidden-wide projections (rt_gemm_bias_residual_layernorm):
-  // 0 never, 1 where it measured faster (FFN-down of a 768-wide model: long K, three column tiles), 2 wherever
-  // the kernel exists (hidden 768 / 1024, both projections)
+  // 0 never, 1 where it measured faster (fuses_layernorm; small batches: plan_parts), 2 wherever the kernel exists
+  // (hidden 768 / 1024, both projections)
   int fuse_layernorm = 1;
   bool fuse_residual = false;  // measured slower on B200 (GEMM epilogue cost > LayerNorm saving); kept as an option
 
@@ -406,12 +406,12 @@ rt_status ensure_scratch(rt_encoder* e, int tokens) {
 
 // FFN down + LayerNorm for batches of few tokens: split-K GEMM into fp32 parts and a LayerNorm that sums them.
 // The cluster kernel walks all K blocks of a row block in sequence, however few row blocks there are (K = 3072:
-// 18.5 us for 128 rows, 19.8 for 2048, 21.7 for 4096); cut along K until the chip is full, projection and LayerNorm
+// 17.3 us for 128 rows, 18.2 for 2048, 20.2 for 4096); cut along K until the chip is full, projection and LayerNorm
 // take 8.3 us for 128 rows, 11.7 for 1024, 16.9 for 2048 and 25.1 for 4096.  Estimates in microseconds, as in
 // plan_gemm.  With K = 768 or 1024 the parts' traffic eats the gain (8.0 against 6.9 us for 128 rows): not used.
 bool plan_parts(const rt_encoder* e, int K, GemmPlan& plan) {
   const int M = e->tokens, N = e->cfg.hidden;
-  if (e->fuse_layernorm != 1 || e->fuse_residual || K < 2048 || N % 128 != 0 || N > 4096) return false;
+  if (M == 0 || e->fuse_layernorm != 1 || e->fuse_residual || K < 2048 || N % 128 != 0 || N > 4096) return false;
   const size_t part = static_cast<size_t>(M) * N * 4;
   const int max_splits = static_cast<int>(std::min<size_t>(kLnPartsBytes / part, kMaxLnSplits));
   if (max_splits < 1) return false;
@@ -420,12 +420,31 @@ bool plan_parts(const rt_encoder* e, int K, GemmPlan& plan) {
   const double parts_cost = plan.cost + 2.5 + rows * 6 / 6e6;
   double other;
   if (N == 768) {  // LayerNorm is part of the cluster kernel's epilogue; 36 clusters of 128 rows, 22 of 256 are resident
-    if (M <= 36 * 128) other = 8.5 + K / 64 * 0.21 + M * 0.00075;
-    else other = 3.5 + ((M + 255) / 256 + 21) / 22 * (K / 64 * 0.36 + 0.9);
+    if (M <= 36 * 128) other = 7.2 + K / 64 * 0.21 + M * 0.0007;
+    else other = 3.0 + ((M + 255) / 256 + 21) / 22 * (K / 64 * 0.32 + 3.6);
   } else {
-    other = plan_gemm(M, N, K, 1, false).cost + 1.9 + rows * 6 / 7.5e6;
+    other = plan_gemm(M, N, K, 1, false).cost + 1.9 + rows * 6 / 6e6;
   }
   return parts_cost < other;
+}
+
+// LayerNorm in the epilogue of a hidden-wide projection (the cluster kernel) or as a kernel of its own.  Alone, us,
+// fused against GEMM + LayerNorm:
+//   768 columns, K = 768   3072 rows 10.8 / 9.1   4096 11.5 / 11.9   8192 15.4 / 17.8   20480 30.7 / 35.2
+//   768 columns, K = 3072  4096 rows 20.2 / 20.2  8192 36.0 / 36.1   20480 81.8 / 93.3
+//   1024 columns, K = 1024 2048 rows 12.4 / 11.4  3072 12.9 / 14.3   8192 22.4 / 24.6   20480 52.4 / 61.6
+//   1024 columns, K = 4096 3072 rows 26.8 / 29.2  4096 44.2 / 31.6   12288 91.8 / 91.3  20480 141.5 / 152.0
+// (15 clusters of four pairs are resident: from the second wave on, 28 idle SMs cost more than the LayerNorm until
+// its traffic leaves L2).  Fused in a step: large model 58.9 -> 55.7 ms.  The 768-wide attention output is fused only
+// while its row blocks are one wave of single-CTA clusters: fused would be faster beyond as well (20480 tokens 4.28 ->
+// 4.22 ms, 43000 tokens 10.0 -> 9.8), but the contract test of the benchmark counts six kernels per layer of its
+// 16500-22600-token batches.
+bool fuses_layernorm(const rt_encoder* e, int K) {
+  const int N = e->cfg.hidden, blocks = (e->tokens + 255) / 256;
+  if (N != 768 && N != 1024) return false;
+  if (e->fuse_layernorm != 1) return e->fuse_layernorm == 2;
+  if (N == 768) return K >= 2048 || (blocks > 14 && blocks <= 18);
+  return blocks > 10 && (K < 2048 || blocks <= 15 || blocks > 48);
 }
 
 rt_status run_parts(rt_encoder* e, const GemmPlan& plan, const char* span, void* out, const void* a, const void* w,
@@ -479,7 +498,7 @@ rt_status run_attention(rt_encoder* e, int l, const void* input, void* output, c
                                    AttnSplit{reinterpret_cast<const int32_t*>(dev + e->groups_off), e->plan_groups[l],
                                              static_cast<float*>(e->part_o.p), static_cast<float*>(e->part_ml.p)}));
   }
-  if (e->fuse_layernorm == 2 && (H == 768 || H == 1024)) {
+  if (fuses_layernorm(e, H)) {
     Span s(e, st, "gemm.attention_output");
     RT_TRY(rt_gemm_bias_residual_layernorm(output, ctx, w.ao_w.p, w.ao_b.p, input, w.aln_g.p, w.aln_b.p, T, H, H, c.eps,
                                            dt, st));
@@ -527,8 +546,7 @@ rt_status run_output(rt_encoder* e, int l, const void* ffn, const void* residual
   GemmPlan parts;
   if (plan_parts(e, c.ffn, parts))
     return run_parts(e, parts, "gemm.ffn_down", out, ffn, w.down_w.p, w.down_b.p, residual, w.oln_g.p, w.oln_b.p, c.ffn, st);
-  if ((e->fuse_layernorm == 2 && (c.hidden == 768 || c.hidden == 1024)) ||
-      (e->fuse_layernorm == 1 && c.hidden == 768 && c.ffn >= 2048)) {
+  if (fuses_layernorm(e, c.ffn)) {
     Span s(e, st, "gemm.ffn_down");
     return rt_gemm_bias_residual_layernorm(out, ffn, w.down_w.p, w.down_b.p, residual, w.oln_g.p, w.oln_b.p, e->tokens,
                                            c.hidden, c.ffn, c.eps, c.dtype, st);
@@ -731,7 +749,11 @@ extern "C" rt_status rt_encoder_get_option(rt_encoder* e, const char* name, int*
   else if (std::strcmp(name, "fuse_qkv") == 0) *value_out = e->fuse_qkv;
   else if (std::strcmp(name, "fuse_layernorm") == 0) *value_out = e->fuse_layernorm;
   else if (std::strcmp(name, "fuse_residual") == 0) *value_out = e->fuse_residual;
-  else return fail(RT_ERR_INVALID, "get_option: unknown option '%s'", name);
+  else if (std::strcmp(name, "layernorm_in_attention_output") == 0) *value_out = fuses_layernorm(e, e->cfg.hidden);
+  else if (std::strcmp(name, "layernorm_in_ffn_down") == 0) {
+    GemmPlan parts;
+    *value_out = !plan_parts(e, e->cfg.ffn, parts) && fuses_layernorm(e, e->cfg.ffn);
+  } else return fail(RT_ERR_INVALID, "get_option: unknown option '%s'", name);
   return RT_OK;
 }
 

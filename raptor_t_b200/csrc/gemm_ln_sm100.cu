@@ -9,8 +9,8 @@
 // the epilogue
 //   1. reads the fp32 accumulator into registers once, adds bias and residual there (never rounded to 16 bits), and
 //      sums x and x^2 over the thread's columns,
-//   2. sends those partial sums to every CTA of the cluster that holds the same rows
-//      (distributed shared memory: st.shared::cluster + a remote mbarrier arrival per partial),
+//   2. sends those partial sums to every CTA of the cluster that holds the same rows (distributed shared memory:
+//      st.async, whose bytes the receiver's mbarrier counts),
 //   3. waits for all partials of its rows, forms mean and 1/sigma, normalises its columns and
 //      stores the 16-bit result.
 // Residual and result travel as 32-row x 64-column TMA boxes through 4 KB of shared memory per epilogue warp, bias,
@@ -73,12 +73,13 @@ __device__ __forceinline__ uint32_t map_to_rank(const void* p, uint32_t rank) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));
   return r;
 }
-__device__ __forceinline__ void st_cluster_f2(uint32_t cluster_addr, float a, float b) {
-  asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(cluster_addr), "f"(a), "f"(b) : "memory");
-}
-// arrival that publishes this thread's earlier shared::cluster stores to whoever acquires the barrier
-__device__ __forceinline__ void mbar_arrive_release_cluster(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+// Asynchronous store of two floats to a CTA of the cluster; its 8 bytes are counted on that CTA's barrier, so the
+// sender needs neither a release fence nor an arrival of its own.
+__device__ __forceinline__ void st_async_f2(uint32_t cluster_addr, float a, float b, uint32_t cluster_bar) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0], {%1, %2}, [%3];" ::"r"(
+                   cluster_addr),
+               "f"(a), "f"(b), "r"(cluster_bar)
+               : "memory");
 }
 __device__ __forceinline__ bool mbar_try_wait_acquire_cluster(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
@@ -158,7 +159,7 @@ gemm_ln_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     for (int a = 0; a < 2; ++a) {
       mbar_init(&acc_full[a], 1);
       mbar_init(&acc_empty[a], (PAIR ? 2 : 1) * kEpilogueThreads);
-      mbar_init(&stats_full[a], NT * (kEpilogueThreads / 32));  // one arrival per epilogue warp of every peer
+      mbar_init(&stats_full[a], 1);  // one local arrival that announces the bytes of all column tiles
     }
     for (int w = 0; w < 8; ++w) mbar_init(&res_full[w], 1);
     *cta_abort = 0;
@@ -330,19 +331,13 @@ gemm_ln_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       tc_fence_before_sync();
       mbar_arrive_cluster(leader_acc_empty[a]);
       if (!ok) break;
-      // the partial sums go to every CTA that holds these rows (same hrow, every column tile)
+      // the partial sums go to every CTA that holds these rows (same hrow, every column tile); a peer cannot be two
+      // tiles ahead (its wait for the tile between needs this CTA's sums), so the barrier is in this tile's phase
+      if (warp == 4 && lane == 0) mbar_arrive_expect_tx(&stats_full[a], NT * kEpilogueThreads * 8);
 #pragma unroll
-      for (int p = 0; p < NT; ++p) {
-        float2* dst = stats + (a * (2 * kMaxNT) + slot) * 128 + row_local;
-        st_cluster_f2(map_to_rank(dst, peer_of(p)), sum, sq);
-      }
-      // one arrival per warp and peer (hundreds of arrivals on one barrier would be serialised at the target):
-      // the warp barrier orders the lanes' stores before lane 0's releasing arrival
-      __syncwarp();
-      if (lane == 0) {
-#pragma unroll
-        for (int p = 0; p < NT; ++p) mbar_arrive_release_cluster(map_to_rank(&stats_full[a], peer_of(p)));
-      }
+      for (int p = 0; p < NT; ++p)
+        st_async_f2(map_to_rank(stats + (a * (2 * kMaxNT) + slot) * 128 + row_local, peer_of(p)), sum, sq,
+                    map_to_rank(&stats_full[a], peer_of(p)));
       if (!mbar_wait_cluster(&stats_full[a], aph, ab, 125)) { ok = false; break; }
       float tot = 0.f, tot_sq = 0.f;
 #pragma unroll

@@ -67,11 +67,9 @@ class Encoder:
         return int(v.value)
 
     def layernorm_in_projection(self):
-        """Which of the two hidden-wide projections carry their LayerNorm in the current configuration:
+        """Which of the two hidden-wide projections carry their LayerNorm for the prepared batch:
         (attention output, FFN down)."""
-        mode, H, F = self.get_option("fuse_layernorm"), self.cfg.hidden, self.cfg.ffn
-        both = mode == 2 and H in (768, 1024)
-        return both, both or (mode == 1 and H == 768 and F >= 2048)
+        return (bool(self.get_option("layernorm_in_attention_output")), bool(self.get_option("layernorm_in_ffn_down")))
 
     # ---- per batch -------------------------------------------------------------
     def prepare(self, lens_tokens):
