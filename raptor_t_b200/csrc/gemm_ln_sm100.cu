@@ -64,7 +64,7 @@ struct LnCfg {
   static constexpr int kWRows = PAIR ? TW / 2 : TW;  // rows of W that one CTA loads
   static constexpr int kStageBytes = kABytes + kWRows * kBK * 2;
   static constexpr int kStages = kStageBytes <= 32 * 1024 ? 5 : 4;
-  static constexpr int kParamBytes = 3 * TW * 2;  // bias, gamma, beta of this CTA's columns
+  static constexpr int kParamBytes = 3 * TW * 4;  // bias, gamma, beta of this CTA's columns, fp32
   static constexpr int kSmemBytes = kStages * kStageBytes + 8 * kBoxBytes + kStatsBytes + kParamBytes + 1024 + 256;
 };
 
@@ -107,6 +107,32 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity
   atomicCAS(ab.global_flag, 0, where);
   return false;
 }
+// packed fp32 pairs: half the issue slots of the scalar forms
+__device__ __forceinline__ uint64_t f2_pack(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 f2_unpack(uint64_t v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ uint64_t f2_add(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t f2_mul(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
 // TMA load into THIS CTA's shared memory whose bytes are counted on the pair leader's barrier
 __device__ __forceinline__ void tma_load_2d_to_leader(void* smem_dst, const CUtensorMap* m, int x, int y, uint32_t leader_bar) {
   asm volatile(
@@ -129,7 +155,7 @@ gemm_ln_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* boxes = smem + kStages * kStageBytes;                             // [8 epilogue warps]
   float2* stats = reinterpret_cast<float2*>(boxes + 8 * kBoxBytes);          // [2][2 * kMaxNT][128]
-  uint16_t* params = reinterpret_cast<uint16_t*>(boxes + 8 * kBoxBytes + kStatsBytes);  // [3][TW]
+  float* params = reinterpret_cast<float*>(boxes + 8 * kBoxBytes + kStatsBytes);  // [3][TW]
   uint64_t* bars = reinterpret_cast<uint64_t*>(boxes + 8 * kBoxBytes + kStatsBytes + Cfg::kParamBytes);
   uint64_t* full = bars;                  // the pair leader's copy is the one in use
   uint64_t* empty = bars + kStages;       // each CTA waits on its own copy
@@ -165,9 +191,9 @@ gemm_ln_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     *cta_abort = 0;
     fence_barrier_init();
   }
-  for (int i = threadIdx.x; i < 3 * TW / 8; i += kThreads) {
-    const uint16_t* src = i < TW / 8 ? bias : i < TW / 4 ? gamma : beta;
-    reinterpret_cast<uint4*>(params)[i] = reinterpret_cast<const uint4*>(src + tile * TW)[i % (TW / 8)];
+  for (int i = threadIdx.x; i < 3 * TW / 2; i += kThreads) {
+    const uint16_t* src = i < TW / 2 ? bias : i < TW ? gamma : beta;
+    reinterpret_cast<float2*>(params)[i] = unpack2<BF16>(reinterpret_cast<const uint32_t*>(src + tile * TW)[i % (TW / 2)]);
   }
   if (warp == 1) {
     if constexpr (PAIR) {
@@ -292,7 +318,7 @@ gemm_ln_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       tc_fence_after_sync();
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + a * kTileN;
       // pass 1: x = acc + bias + residual in registers; partial sums of x and x^2
-      float sum = 0.f, sq = 0.f;
+      uint64_t sum2 = 0, sq2 = 0;  // packed pairs of fp32
       uint32_t x[128];
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
@@ -306,19 +332,20 @@ gemm_ln_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 #pragma unroll
           for (int q = 0; q < 8; ++q) {
             const uint4 r4 = *reinterpret_cast<const uint4*>(line + ((q ^ swz) << 4));
-            const uint4 b4 = *reinterpret_cast<const uint4*>(params + b * 64 + q * 8);
-            const uint32_t rw[4] = {r4.x, r4.y, r4.z, r4.w}, bw[4] = {b4.x, b4.y, b4.z, b4.w};
+            const ulonglong2* bv = reinterpret_cast<const ulonglong2*>(params + b * 64 + q * 8);
+            const ulonglong2 b01 = bv[0], b23 = bv[1];
+            const uint64_t bb[4] = {b01.x, b01.y, b23.x, b23.y};
+            const uint32_t rw[4] = {r4.x, r4.y, r4.z, r4.w};
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-              const float2 bb = unpack2<BF16>(bw[j]);
               const float2 rr = unpack2<BF16>(rw[j]);
               uint32_t* v = x + i * 64 + q * 8 + 2 * j;
-              const float x0 = __uint_as_float(v[0]) + bb.x + rr.x;
-              const float x1 = __uint_as_float(v[1]) + bb.y + rr.y;
-              sum += x0 + x1;
-              sq = fmaf(x0, x0, fmaf(x1, x1, sq));
-              v[0] = __float_as_uint(x0);
-              v[1] = __float_as_uint(x1);
+              const uint64_t y = f2_add(f2_add(f2_pack(__uint_as_float(v[0]), __uint_as_float(v[1])), bb[j]), f2_pack(rr.x, rr.y));
+              sum2 = f2_add(sum2, y);
+              sq2 = f2_fma(y, y, sq2);
+              const float2 f = f2_unpack(y);
+              v[0] = __float_as_uint(f.x);
+              v[1] = __float_as_uint(f.y);
             }
           }
           if (i == 0 && set + 2 < kBoxes) {
@@ -327,6 +354,8 @@ gemm_ln_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           }
         }
       }
+      const float2 sums = f2_unpack(sum2), sqs = f2_unpack(sq2);
+      const float sum = sums.x + sums.y, sq = sqs.x + sqs.y;
       // the accumulator is in registers: the tile after the next may overwrite it
       tc_fence_before_sync();
       mbar_arrive_cluster(leader_acc_empty[a]);
@@ -351,6 +380,7 @@ gemm_ln_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       const float rstd = rsqrtf(var + eps);
       // pass 2: normalise this thread's columns, store them box by box
       const int row0 = row0_of(t);
+      const uint64_t neg_mean = f2_pack(-mean, -mean), rstd2 = f2_pack(rstd, rstd);
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
         const int b = set + 2 * i;
@@ -361,16 +391,17 @@ gemm_ln_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           }
 #pragma unroll
           for (int q = 0; q < 8; ++q) {
-            const uint4 g4 = *reinterpret_cast<const uint4*>(params + TW + b * 64 + q * 8);
-            const uint4 e4 = *reinterpret_cast<const uint4*>(params + 2 * TW + b * 64 + q * 8);
-            const uint32_t gw[4] = {g4.x, g4.y, g4.z, g4.w}, ew[4] = {e4.x, e4.y, e4.z, e4.w};
+            const ulonglong2* gv = reinterpret_cast<const ulonglong2*>(params + TW + b * 64 + q * 8);
+            const ulonglong2* ev = reinterpret_cast<const ulonglong2*>(params + 2 * TW + b * 64 + q * 8);
+            const ulonglong2 g01 = gv[0], g23 = gv[1], e01 = ev[0], e23 = ev[1];
+            const uint64_t gg[4] = {g01.x, g01.y, g23.x, g23.y}, ee[4] = {e01.x, e01.y, e23.x, e23.y};
             uint32_t o[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-              const float2 gg = unpack2<BF16>(gw[j]), ee = unpack2<BF16>(ew[j]);
               const uint32_t* v = x + i * 64 + q * 8 + 2 * j;
-              o[j] = pack2<BF16>((__uint_as_float(v[0]) - mean) * rstd * gg.x + ee.x,
-                                 (__uint_as_float(v[1]) - mean) * rstd * gg.y + ee.y);
+              const uint64_t y = f2_mul(f2_add(f2_pack(__uint_as_float(v[0]), __uint_as_float(v[1])), neg_mean), rstd2);
+              const float2 f = f2_unpack(f2_fma(y, gg[j], ee[j]));
+              o[j] = pack2<BF16>(f.x, f.y);
             }
             *reinterpret_cast<uint4*>(line + ((q ^ swz) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
           }
