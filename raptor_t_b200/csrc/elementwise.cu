@@ -333,7 +333,10 @@ __global__ void __launch_bounds__(256) qkv_transpose_kernel(const T* __restrict_
 }
 
 // ---------------------------------------------------------------------------
-// embeddings: fp32 tables, one warp per token, same statistics as LayerNorm.
+// embeddings: fp32 tables, one warp per token, same statistics as LayerNorm.  Bound by the gather of the word rows
+// from HBM: a warp reads its rows in contiguous 512-byte pieces, all of them in flight at once (NV per table), and
+// walks the tokens with a grid stride, so that gamma and beta are staged in shared memory once per CTA.  20480 tokens of 768:
+// 24.6 us (44.7 with 16-byte loads at a stride of 32 and parameters read word by word), 76000 of 1024: 92 (207).
 // ---------------------------------------------------------------------------
 template <typename T, int NV>
 __global__ void __launch_bounds__(256) embeddings_kernel(T* __restrict__ out, const int32_t* __restrict__ ids,
@@ -343,60 +346,66 @@ __global__ void __launch_bounds__(256) embeddings_kernel(T* __restrict__ out, co
                                                          const float* __restrict__ type, const float* __restrict__ gamma,
                                                          const float* __restrict__ beta, int tokens, int hidden,
                                                          float eps) {
+  __shared__ float4 s_gamma[32 * NV], s_beta[32 * NV];
   RT_PDL_LAUNCH_DEPENDENTS();
   RT_PDL_WAIT();
+  for (int i = threadIdx.x; i < hidden; i += blockDim.x) {  // scalar: the parameters need no alignment
+    reinterpret_cast<float*>(s_gamma)[i] = gamma[i];
+    reinterpret_cast<float*>(s_beta)[i] = beta[i];
+  }
+  __syncthreads();
   const int lane = threadIdx.x & 31;
-  const int warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (warp >= tokens) return;
-  const int vecs = hidden >> 3;
-  const size_t wi = static_cast<size_t>(ids[warp]) * hidden;
-  const size_t pi = static_cast<size_t>(pos_ids ? pos_ids[warp] : 0) * hidden;
-  const size_t ti = static_cast<size_t>(type_ids ? type_ids[warp] : 0) * hidden;
-  float v[NV][8];
-  float sum = 0.f;
-#pragma unroll
-  for (int i = 0; i < NV; ++i) {
-    const int c = lane + 32 * i;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) v[i][k] = 0.f;
-    if (c < vecs) {
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        const float4 a = *reinterpret_cast<const float4*>(word + wi + c * 8 + half * 4);
-        const float4 p = *reinterpret_cast<const float4*>(pos + pi + c * 8 + half * 4);
-        const float4 t = *reinterpret_cast<const float4*>(type + ti + c * 8 + half * 4);
-        v[i][half * 4 + 0] = a.x + t.x + p.x;
-        v[i][half * 4 + 1] = a.y + t.y + p.y;
-        v[i][half * 4 + 2] = a.z + t.z + p.z;
-        v[i][half * 4 + 3] = a.w + t.w + p.w;
-      }
-#pragma unroll
-      for (int k = 0; k < 8; ++k) sum += v[i][k];
-    }
-  }
+  const int warps = gridDim.x * (blockDim.x >> 5);
+  const int vecs = hidden >> 2;
   const float inv_h = 1.0f / static_cast<float>(hidden);
-  const float mean = warp_sum(sum) * inv_h;
-  float sq = 0.f;
+  for (int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); t < tokens; t += warps) {
+    const float4* wr = reinterpret_cast<const float4*>(word + static_cast<size_t>(ids[t]) * hidden);
+    const float4* pr = reinterpret_cast<const float4*>(pos + static_cast<size_t>(pos_ids ? pos_ids[t] : 0) * hidden);
+    const float4* tr = reinterpret_cast<const float4*>(type + static_cast<size_t>(type_ids ? type_ids[t] : 0) * hidden);
+    float4 v[NV], pv[NV], tv[NV];
 #pragma unroll
-  for (int i = 0; i < NV; ++i) {
-    if (lane + 32 * i < vecs) {
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        const float d = v[i][k] - mean;
-        sq += d * d;
+    for (int i = 0; i < NV; ++i) {
+      const int c = lane + 32 * i;
+      if (c < vecs) {
+        v[i] = wr[c];
+        pv[i] = pr[c];
+        tv[i] = tr[c];
       }
     }
-  }
-  const float rstd = rsqrtf(warp_sum(sq) * inv_h + eps);
-  uint4* orow = reinterpret_cast<uint4*>(out + static_cast<size_t>(warp) * hidden);
+    float sum = 0.f;
 #pragma unroll
-  for (int i = 0; i < NV; ++i) {
-    const int c = lane + 32 * i;
-    if (c < vecs) {
-      float o[8];
+    for (int i = 0; i < NV; ++i) {
+      if (lane + 32 * i < vecs) {
+        v[i].x = v[i].x + tv[i].x + pv[i].x;
+        v[i].y = v[i].y + tv[i].y + pv[i].y;
+        v[i].z = v[i].z + tv[i].z + pv[i].z;
+        v[i].w = v[i].w + tv[i].w + pv[i].w;
+        sum += (v[i].x + v[i].y) + (v[i].z + v[i].w);
+      }
+    }
+    const float mean = warp_sum(sum) * inv_h;
+    float sq = 0.f;
 #pragma unroll
-      for (int k = 0; k < 8; ++k) o[k] = (v[i][k] - mean) * rstd * gamma[c * 8 + k] + beta[c * 8 + k];
-      orow[c] = Vec8<T>::pack(o);
+    for (int i = 0; i < NV; ++i) {
+      if (lane + 32 * i < vecs) {
+        v[i].x -= mean;
+        v[i].y -= mean;
+        v[i].z -= mean;
+        v[i].w -= mean;
+        sq += (v[i].x * v[i].x + v[i].y * v[i].y) + (v[i].z * v[i].z + v[i].w * v[i].w);
+      }
+    }
+    const float rstd = rsqrtf(warp_sum(sq) * inv_h + eps);
+    T* orow = out + static_cast<size_t>(t) * hidden;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const int c = lane + 32 * i;
+      if (c < vecs) {
+        const float4 g = s_gamma[c], b = s_beta[c];
+        const float o[4] = {v[i].x * rstd * g.x + b.x, v[i].y * rstd * g.y + b.y, v[i].z * rstd * g.z + b.z,
+                            v[i].w * rstd * g.w + b.w};
+        pack4(o, orow + 4 * c);
+      }
     }
   }
 }
@@ -542,18 +551,18 @@ extern "C" rt_status rt_embeddings(void* out, const int32_t* ids, const int32_t*
   RT_REQUIRE(aligned16(out) && aligned16(word) && aligned16(pos) && aligned16(type), RT_ERR_INVALID,
              "embeddings: pointers must be 16-byte aligned");
   if (tokens == 0) return RT_OK;
-  const int nv = (hidden / 8 + 31) / 32;
+  const int nv = (hidden / 4 + 63) / 64;  // pairs of 512-byte pieces per row
   const int threads = 256, wpb = 8;
-  const int blocks = (tokens + wpb - 1) / wpb;
+  const int blocks = std::min((tokens + wpb - 1) / wpb, sm_count() * 4);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
 #define RT_EMB(T, NV)                                                                                          \
   launch_kernel(embeddings_kernel<T, NV>, dim3(blocks), dim3(threads), 0, st, (T*)out, ids, pos_ids, type_ids, \
                 (const float*)word, (const float*)pos, (const float*)type, (const float*)gamma,                \
                 (const float*)beta, tokens, hidden, eps)
   if (dtype == RT_F16) {
-    switch (nv) { case 1: RT_EMB(__half, 1); break; case 2: RT_EMB(__half, 2); break; case 3: RT_EMB(__half, 3); break; default: RT_EMB(__half, 4); }
+    switch (nv) { case 1: RT_EMB(__half, 2); break; case 2: RT_EMB(__half, 4); break; case 3: RT_EMB(__half, 6); break; default: RT_EMB(__half, 8); }
   } else if (dtype == RT_BF16) {
-    switch (nv) { case 1: RT_EMB(__nv_bfloat16, 1); break; case 2: RT_EMB(__nv_bfloat16, 2); break; case 3: RT_EMB(__nv_bfloat16, 3); break; default: RT_EMB(__nv_bfloat16, 4); }
+    switch (nv) { case 1: RT_EMB(__nv_bfloat16, 2); break; case 2: RT_EMB(__nv_bfloat16, 4); break; case 3: RT_EMB(__nv_bfloat16, 6); break; default: RT_EMB(__nv_bfloat16, 8); }
   } else {
     return fail(RT_ERR_INVALID, "embeddings: unknown dtype %d", dtype);
   }
