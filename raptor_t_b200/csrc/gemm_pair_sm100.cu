@@ -1,8 +1,9 @@
 // Two-CTA (cta_group::2) variant of the tcgen05 GEMM: a cluster of two CTAs on neighbouring
-// SMs computes one 256 x 256 output tile.  Each CTA loads its own 128 rows of A and its own
-// 128 rows of W per 64-wide K slice (32 KB instead of the 48 KB a single-CTA 128 x 256 tile
-// needs for the same MMA work), the leader CTA issues one M=256 N=256 K=16 MMA for the pair,
-// and each CTA drains its own 128 accumulator rows.  The single-CTA kernel is bound by the
+// SMs computes one output tile of 256 rows and 64, 128, 192 or 256 columns (one launch may mix whole waves of
+// 256 columns with narrower tiles for the rest, see plan_gemm).  Each CTA loads its own 128 rows of A and half of
+// the tile's rows of W per 64-wide K slice (256 columns: 32 KB instead of the 48 KB a single-CTA 128 x 256 tile
+// needs for the same MMA work), the leader CTA issues the M=256 K=16 MMAs for the pair, and each CTA drains its own
+// 128 accumulator rows.  The single-CTA kernel is bound by the
 // L2 -> shared-memory traffic of its operand tiles; the pair moves a third less per FLOP.
 //
 // No TMA multicast is used: both CTAs issue plain (cta_group::2) loads of their own tiles
@@ -254,7 +255,7 @@ rt_status launch_pair(void* c, const void* a, const void* w, const void* bias, i
 
 }  // namespace
 
-// Entry used by rt_gemm / rt_gemm_qkv when the shape suits 256 x 256 pair tiles.
+// main_tiles tiles of 256 columns, the rest of the output in tiles of tail_w (GemmPlan).
 rt_status gemm_pair_dispatch(void* c, const void* a, const void* w, const void* bias, int M, int N, int K, int epi,
                              bool bf16, cudaStream_t st, const gemm_detail::QkvEpilogue& qkv, int main_tiles, int tail_w) {
   switch (epi) {

@@ -369,6 +369,11 @@ class MetaData {
   // layers/metadata.cpp:6-18: once per batch, before the forward pass
   void update_meta_data(int64_t total_seq_len, int64_t to_select_index_len, int64_t to_select_index_position_len,
                         std::vector<int> seq_len_info) {
+    // the uploads read host memory of this batch only: a graph would replay them from recycled memory
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(at::cuda::getCurrentCUDAStream().stream(), &capturing) != cudaSuccess ||
+        capturing != cudaStreamCaptureStatusNone)
+      throw std::runtime_error("update_meta_data: the stream is being captured");
     TensorSet* ts = TensorSet::get_instance();
     ts->update_tensor_set(total_seq_len, to_select_index_len, to_select_index_position_len, seq_len_info);
     const std::vector<int32_t> lens = ts->lens_tokens();

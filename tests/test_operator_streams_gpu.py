@@ -48,3 +48,13 @@ def test_batches_in_a_loop_match_single_batches(two_streams):
         assert torch.equal(out, want[i % len(batches)]), i
     md.terminate_thread()
     ops.check_device()
+
+
+def test_update_meta_data_refuses_a_capturing_stream():
+    from raptor_t_b200 import compiled
+    md = compiled.load().MetaData()
+    g = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(g):
+        with pytest.raises(RuntimeError, match="captured"):
+            md.update_meta_data(1024, 17, 100, [0, 16])
