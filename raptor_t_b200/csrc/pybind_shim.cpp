@@ -99,6 +99,79 @@ void timed(InfoMap& info, const char* key, F&& fn) {
 }
 
 // ---------------------------------------------------------------------------------------------
+// Order of the calls that touch process-wide buffers (the TensorSet): each waits on its stream for the one before it,
+// whatever stream that ran on, by an event behind the last use.  Calls on one stream are in order anyway (the wait
+// costs the host well under a microsecond and the device nothing); the host waits for nothing.
+// ---------------------------------------------------------------------------------------------
+class SharedOrder {
+ public:
+  static SharedOrder& get() {
+    static SharedOrder o;
+    return o;
+  }
+  void begin(const c10::cuda::CUDAStream& s) {
+    if (first_ && *first_ != s) several_streams_ = true;
+    first_ = first_ ? first_ : s;
+    if (!last_) return;
+    if (capturing(s)) {
+      wait_on_host();  // a graph cannot wait for work outside it
+      return;
+    }
+    if (cudaStreamWaitEvent(s.stream(), last_, 0) != cudaSuccess)
+      throw std::runtime_error("raptor_t: cannot order the call behind the previous one");
+  }
+  // noexcept: runs while an exception of the call is on its way, too
+  void end(const c10::cuda::CUDAStream& s) noexcept {
+    if (capturing(s)) {  // replays come whenever the caller wants them: no event stands behind them
+      captured_ = true;
+      return;
+    }
+    cudaEvent_t& e = events_[s.device_index() & 63];
+    if (!e) cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
+    if (cudaEventRecord(e, s.stream()) == cudaSuccess) last_ = e;
+    else cudaDeviceSynchronize();
+  }
+  // before a shared buffer is given back to the stream it was allocated on, which other streams' uses are not part of
+  void before_release() {
+    if (several_streams_ && last_) wait_on_host();
+  }
+  // before the next batch: replays of a captured call may run on any stream
+  void before_batch() {
+    if (captured_ && cudaDeviceSynchronize() != cudaSuccess)
+      throw std::runtime_error("raptor_t: waiting for captured calls failed");
+  }
+
+ private:
+  static bool capturing(const c10::cuda::CUDAStream& s) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(s.stream(), &st) != cudaSuccess || st != cudaStreamCaptureStatusNone;
+  }
+  void wait_on_host() const {
+    // the event was recorded outside any capture; the relaxed mode keeps another stream's capture valid
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    const cudaError_t e = cudaEventSynchronize(last_);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (e != cudaSuccess) throw std::runtime_error("raptor_t: waiting for the previous call failed");
+  }
+  cudaEvent_t events_[64] = {};  // one per device
+  cudaEvent_t last_ = nullptr;   // behind the latest use
+  std::optional<c10::cuda::CUDAStream> first_;
+  bool several_streams_ = false, captured_ = false;
+};
+
+// One use of the shared buffers on the current stream.
+class SharedUse {
+ public:
+  SharedUse() : stream_(at::cuda::getCurrentCUDAStream()) { SharedOrder::get().begin(stream_); }
+  ~SharedUse() { SharedOrder::get().end(stream_); }
+  SharedUse(const SharedUse&) = delete;
+
+ private:
+  c10::cuda::CUDAStream stream_;
+};
+
+// ---------------------------------------------------------------------------------------------
 // TensorSet: process-wide scratch buffers resized per batch (layers/tensor_set.h:36-65)
 // ---------------------------------------------------------------------------------------------
 class TensorSet {
@@ -123,8 +196,10 @@ class TensorSet {
   // [total_seq_len, cols] view of the named buffer; (re)allocated when the batch or model grows
   torch::Tensor get(const std::string& name, int64_t cols, torch::ScalarType dtype) {
     auto& t = tensors_[name];
-    if (!t.defined() || t.size(0) < total_seq_len_ || t.size(1) != cols || t.scalar_type() != dtype)
+    if (!t.defined() || t.size(0) < total_seq_len_ || t.size(1) != cols || t.scalar_type() != dtype) {
+      if (t.defined()) SharedOrder::get().before_release();
       t = torch::empty({std::max<int64_t>(total_seq_len_, 1), cols}, torch::dtype(dtype).device(torch::kCUDA));
+    }
     return t.narrow(0, 0, total_seq_len_);
   }
   torch::Tensor get_tensor(const std::string& name) {
@@ -284,6 +359,7 @@ class BertAttention {
                bool kernel_fusion, bool /*balanced*/) {
     require_cuda(input_tensor, "input_tensor");
     require_cuda(output, "output");
+    const SharedUse use;
     TensorSet* ts = TensorSet::get_instance();
     const int T = static_cast<int>(input_tensor.size(0));
     const auto st_dtype = input_tensor.scalar_type();
@@ -374,6 +450,7 @@ class MetaData {
     if (cudaStreamIsCapturing(at::cuda::getCurrentCUDAStream().stream(), &capturing) != cudaSuccess ||
         capturing != cudaStreamCaptureStatusNone)
       throw std::runtime_error("update_meta_data: the stream is being captured");
+    SharedOrder::get().before_batch();
     TensorSet* ts = TensorSet::get_instance();
     ts->update_tensor_set(total_seq_len, to_select_index_len, to_select_index_position_len, seq_len_info);
     const std::vector<int32_t> lens = ts->lens_tokens();
@@ -465,6 +542,7 @@ class BertOutput {
     require_cuda(output, "output");
     const int T = static_cast<int>(hidden_states.size(0));
     void* st = stream_of_current();
+    const SharedUse use;
     torch::Tensor dense = TensorSet::get_instance()->get("dense_out", hidden_, hidden_states.scalar_type());
     check(rt_gemm(dense.data_ptr(), hidden_states.data_ptr(), w_.data_ptr(), nullptr, T, hidden_, ffn_, RT_EPI_NONE, dtype_,
                   st));

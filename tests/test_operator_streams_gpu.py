@@ -58,3 +58,65 @@ def test_update_meta_data_refuses_a_capturing_stream():
     with torch.cuda.graph(g):
         with pytest.raises(RuntimeError, match="captured"):
             md.update_meta_data(1024, 17, 100, [0, 16])
+
+
+def _model_and_batches(heads, lens_of_batches):
+    from raptor_t_b200 import compiled, metadata
+    from raptor_t_b200.modeling_bert import BertModelNoPooler
+    raptor_t = compiled.load()
+    cfg = oracle.EncoderConfig(hidden=64 * heads, heads=heads, ffn=256, layers=2, max_pos=4096, vocab=97)
+    P = oracle.make_weights(cfg, seed=3, nonzero_bias=True)
+    model = BertModelNoPooler.from_weights(P, cfg.hidden, cfg.heads, cfg.ffn, cfg.layers, torch.float16, True,
+                                           backend=raptor_t)
+    md = raptor_t.MetaData()
+    batches = []
+    for i, lens in enumerate(lens_of_batches):
+        prefix, total, _, _ = metadata.generate_data_metainfo(lens, 64, 160, cfg.heads)
+        gen = torch.Generator(device="cuda").manual_seed(i)
+        batches.append(dict(T=sum(lens), prefix=prefix, total=total,
+                            ids=torch.randint(0, 97, (sum(lens),), device="cuda", generator=gen, dtype=torch.int32),
+                            pos=torch.cat([torch.arange(n, dtype=torch.int32, device="cuda") for n in lens]),
+                            prefix_dev=torch.tensor(prefix, dtype=torch.int32, device="cuda")))
+    torch.cuda.synchronize()
+
+    def update(b):
+        md.update_meta_data(b["T"], b["prefix"][-1] + 1, b["total"], b["prefix"])
+
+    def forward(b):
+        return model(b["ids"], b["T"], 160, b["prefix"], b["prefix_dev"], position_ids=b["pos"], test_info={})[0]
+
+    return md, batches, update, forward
+
+
+def _wanted(batches, update, forward):
+    want = []
+    for b in batches:
+        update(b)
+        want.append(forward(b).clone())
+        torch.cuda.synchronize()
+    return want
+
+
+def test_batches_on_alternating_streams():
+    """The operator objects share scratch: a batch on another stream comes behind the one before it, also where the
+    scratch grows there, and nobody synchronises."""
+    from raptor_t_b200 import ops
+    md, batches, update, forward = _model_and_batches(3, [[256], [512, 1984], [4096, 1024], [320], [1024] * 7])
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    got, done = [], []
+    for i in range(4 * len(batches)):  # 5 batches, 2 streams: every batch comes on both
+        b, s = batches[i % len(batches)], streams[i % 2]
+        update(b)
+        with torch.cuda.stream(s):
+            if i % 4 == 1:
+                torch.cuda._sleep(20_000_000)  # this stream is late: the next batch must not overtake it
+            got.append(forward(b))
+            done.append(s.record_event())
+    done[-1].synchronize()
+    assert all(e.query() for e in done)
+    torch.cuda.synchronize()
+    for i, w in enumerate(_wanted(batches, update, forward)):
+        for out in got[i::len(batches)]:
+            assert torch.equal(out, w), i
+    md.terminate_thread()
+    ops.check_device()
