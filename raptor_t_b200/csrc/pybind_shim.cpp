@@ -99,7 +99,7 @@ void timed(InfoMap& info, const char* key, F&& fn) {
 }
 
 // ---------------------------------------------------------------------------------------------
-// Order of the calls that touch process-wide buffers (the TensorSet): each waits on its stream for the one before it,
+// Order of the calls that touch process-wide buffers (TensorSet, the batch's maps): each waits on its stream for the one before it,
 // whatever stream that ran on, by an event behind the last use.  Calls on one stream are in order anyway (the wait
 // costs the host well under a microsecond and the device nothing); the host waits for nothing.
 // ---------------------------------------------------------------------------------------------
@@ -240,24 +240,19 @@ class BertAttention;
 struct LayerRegistry {
   std::mutex mu;
   std::vector<BertAttention*> layers;
+  // Maps of the current batch, written in place by update_meta_data and read by the calls, all under a SharedUse.
   torch::Tensor block_seq;  // per packed 64-token block {first token of its sequence, length}: the fused QKV epilogue's map
   torch::Tensor seq_prefix; // int32 [B+1] block offsets of the sequences (device): the pooler's "first token" map
-  std::optional<c10::cuda::CUDAStream> upload_stream;  // both tensors belong to it
-  cudaEvent_t upload_done = nullptr;
+  int n_seq = 0;
 
-  void uploaded_on(const c10::cuda::CUDAStream& s) {
-    if (!upload_done) cudaEventCreateWithFlags(&upload_done, cudaEventDisableTiming);
-    cudaEventRecord(upload_done, s.stream());
-    upload_stream = s;
-  }
-  // Before the current stream reads them: a stream other than the uploading one waits for the copies and keeps
-  // the tensors' memory from being reused under its kernels.
-  void use_on_current_stream() {
-    const auto s = at::cuda::getCurrentCUDAStream();
-    if (!upload_stream || s == *upload_stream) return;
-    cudaStreamWaitEvent(s.stream(), upload_done, 0);
-    block_seq.record_stream(s);
-    seq_prefix.record_stream(s);
+  // from pinned memory, so that the copy does not wait for the previous batch's kernels
+  static void upload(torch::Tensor& to, std::vector<int32_t>& v) {
+    const auto n = static_cast<int64_t>(v.size());
+    if (!to.defined() || to.numel() < n || to.device().index() != c10::cuda::current_device()) {
+      if (to.defined()) SharedOrder::get().before_release();
+      to = torch::empty({std::max<int64_t>(2 * n, 64)}, torch::dtype(torch::kInt32).device(torch::kCUDA));
+    }
+    if (n > 0) to.narrow(0, 0, n).copy_(torch::from_blob(v.data(), {n}, torch::kInt32).pin_memory(), /*non_blocking=*/true);
   }
   static LayerRegistry& get() {
     static LayerRegistry r;
@@ -368,7 +363,6 @@ class BertAttention {
     torch::Tensor dense = ts->get("dense_out", hidden_, st_dtype);
     void* st = stream_of_current();
     auto& reg = LayerRegistry::get();
-    reg.use_on_current_stream();
     if (kernel_fusion && reg.block_seq.defined() && info.find("add_bias_and_transpose_kernel") == info.end()) {
       check(rt_gemm_qkv(q.data_ptr(), k.data_ptr(), v.data_ptr(), input_tensor.data_ptr(), qkv_w_.data_ptr(),
                         qkv_b_.data_ptr(), reg.block_seq.data_ptr<int32_t>(), T, heads_, hidden_, 0.125f, dtype_, st));
@@ -471,14 +465,10 @@ class MetaData {
     }
     auto& reg = LayerRegistry::get();
     std::lock_guard<std::mutex> lk(reg.mu);
-    // from pinned memory, so that the copies do not wait for the previous batch's kernels
-    auto upload = [](std::vector<int32_t>& v) {
-      return torch::from_blob(v.data(), {static_cast<int64_t>(v.size())}, torch::kInt32).pin_memory()
-          .to(torch::kCUDA, /*non_blocking=*/true);
-    };
-    reg.block_seq = upload(bs);
-    reg.seq_prefix = upload(seq_len_info);
-    reg.uploaded_on(at::cuda::getCurrentCUDAStream());
+    const SharedUse use;
+    LayerRegistry::upload(reg.block_seq, bs);
+    LayerRegistry::upload(reg.seq_prefix, seq_len_info);
+    reg.n_seq = static_cast<int>(lens.size());
     for (BertAttention* l : reg.layers)
       if (l) l->kick(lens, device);
   }
@@ -574,10 +564,10 @@ class BertPooler {
     require_cuda(output, "output");
     auto& reg = LayerRegistry::get();
     if (!reg.seq_prefix.defined()) throw std::runtime_error("raptor_t: BertPooler called before MetaData.update_meta_data");
-    reg.use_on_current_stream();
+    const SharedUse use;
     if (output.scalar_type() != torch::kFloat32) throw std::runtime_error("raptor_t: BertPooler writes a float32 output");
     check(rt_pooler(output.data_ptr<float>(), input_tensor.data_ptr(), reg.seq_prefix.data_ptr<int32_t>(),
-                    static_cast<int>(reg.seq_prefix.numel()) - 1, w_.data_ptr(), b_.data_ptr(), hidden_, dtype_,
+                    reg.n_seq, w_.data_ptr(), b_.data_ptr(), hidden_, dtype_,
                     stream_of_current()));
     return output;
   }

@@ -120,3 +120,37 @@ def test_batches_on_alternating_streams():
             assert torch.equal(out, w), i
     md.terminate_thread()
     ops.check_device()
+
+
+def test_captured_forward_replays():
+    """A warm model captures into a graph on another stream than the metadata was uploaded on, and the next batch's
+    metadata waits for replays in flight."""
+    from raptor_t_b200 import ops
+    md, batches, update, forward = _model_and_batches(2, [[832, 1024], [4096, 512]])
+    want = _wanted(batches, update, forward)
+    b = batches[0]
+    update(b)
+    forward(b)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        out = forward(b)
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, want[0])
+    b["ids"].copy_(b["ids"].flip(0))
+    flipped = forward(b).clone()
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, flipped) and not torch.equal(flipped, want[0])
+    s = torch.cuda.Stream()
+    with torch.cuda.stream(s):
+        torch.cuda._sleep(20_000_000)
+        g.replay()
+        done = s.record_event()
+    update(batches[1])
+    assert done.query()
+    assert torch.equal(forward(batches[1]), want[1])
+    torch.cuda.synchronize()
+    assert torch.equal(out, flipped)
+    md.terminate_thread()
+    ops.check_device()
