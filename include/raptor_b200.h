@@ -171,9 +171,11 @@ typedef struct rt_attn_plan rt_attn_plan;
 rt_status rt_attn_plan_create(const rt_config* cfg, const int32_t* lens_tokens, int n_seq,
                               const int32_t* kv_ptr_host, const int32_t* kv_idx_host, int n_ctas,
                               int split_entries, void* stream, rt_attn_plan** plan_out);
+/* waits for the plan's device, whichever device is current */
 rt_status rt_attn_plan_destroy(rt_attn_plan* plan);
 /* The same without waiting for the device: the plan's memory is given back once the work queued on `stream` so
- * far has run.  For callers that used the plan on that stream only. */
+ * far has run.  `stream` is a live stream of the plan's device (NULL: its default stream) that is behind every use
+ * of the plan. */
 rt_status rt_attn_plan_destroy_on(rt_attn_plan* plan, void* stream);
 /* issued key/value block loads (work-list entries) and useful visits, for roofline accounting */
 rt_status rt_attn_plan_stats(const rt_attn_plan* plan, int64_t* entries_out, int64_t* visits_out,

@@ -749,6 +749,7 @@ rt_status plan_pool(cudaMemPool_t* out) {
 
 struct rt_attn_plan {
   AttnPlanHost host;
+  int device = 0;  // of the memory and of the kernels that read it
   uint8_t* dev = nullptr;
   size_t items_off = 0, entries_off = 0, cta_off = 0, groups_off = 0, part_o_off = 0, part_ml_off = 0, bytes = 0;
   int n_ctas = 0;
@@ -778,6 +779,7 @@ extern "C" rt_status rt_attn_plan_create(const rt_config* cfg, const int32_t* le
     return s;
   }
   p->n_ctas = n_ctas;
+  cudaGetDevice(&p->device);
   auto align = [](size_t x) { return (x + 255) & ~size_t(255); };
   p->items_off = 0;
   p->entries_off = align(p->host.items.size() * sizeof(AttnItem));
@@ -816,21 +818,45 @@ extern "C" rt_status rt_attn_plan_create(const rt_config* cfg, const int32_t* le
   return RT_OK;
 }
 
+namespace {
+// The device of a plan, current for the length of a call.
+struct OnDevice {
+  int before = 0;
+  cudaError_t status;
+  explicit OnDevice(int device) {
+    status = cudaGetDevice(&before);
+    if (status == cudaSuccess && before != device) status = cudaSetDevice(device);
+  }
+  ~OnDevice() { cudaSetDevice(before); }
+};
+}  // namespace
+
 extern "C" rt_status rt_attn_plan_destroy(rt_attn_plan* p) {
   if (!p) return RT_OK;
+  cudaError_t e = cudaSuccess;
   if (p->dev) {
-    cudaDeviceSynchronize();  // kernels of any stream may still read it
-    cudaFree(p->dev);
+    // kernels of any stream may still read it, and cudaFree waits for none where the memory is a pool's; memory that
+    // could not be waited for stays allocated
+    OnDevice on(p->device);
+    e = on.status;
+    if (e == cudaSuccess) e = cudaDeviceSynchronize();
+    if (e == cudaSuccess) e = cudaFree(p->dev);
   }
   delete p;
+  if (e != cudaSuccess) return fail(RT_ERR_CUDA, "attn_plan_destroy: %s", cudaGetErrorString(e));
   return RT_OK;
 }
 
 extern "C" rt_status rt_attn_plan_destroy_on(rt_attn_plan* p, void* stream) {
   if (!p) return RT_OK;
-  cudaError_t e = p->dev ? cudaFreeAsync(p->dev, static_cast<cudaStream_t>(stream)) : cudaSuccess;
+  if (p->dev) {
+    OnDevice on(p->device);  // the default stream is the plan's device's, too
+    if (on.status != cudaSuccess || cudaFreeAsync(p->dev, static_cast<cudaStream_t>(stream)) != cudaSuccess) {
+      cudaGetLastError();  // handled: the next launch must not report it
+      return rt_attn_plan_destroy(p);
+    }
+  }
   delete p;
-  if (e != cudaSuccess) return fail(RT_ERR_CUDA, "attn_plan_destroy_on: %s", cudaGetErrorString(e));
   return RT_OK;
 }
 

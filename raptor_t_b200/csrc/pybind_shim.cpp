@@ -38,6 +38,7 @@
 #include <optional>
 #include <stdexcept>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/raptor_b200.h"
@@ -166,6 +167,7 @@ class SharedUse {
   SharedUse() : stream_(at::cuda::getCurrentCUDAStream()) { SharedOrder::get().begin(stream_); }
   ~SharedUse() { SharedOrder::get().end(stream_); }
   SharedUse(const SharedUse&) = delete;
+  const c10::cuda::CUDAStream& stream() const { return stream_; }
 
  private:
   c10::cuda::CUDAStream stream_;
@@ -286,7 +288,7 @@ class BertAttention {
     reg.layers.push_back(this);
   }
   ~BertAttention() {
-    drop_plan();
+    drop_plan(nullptr);
     auto& reg = LayerRegistry::get();
     std::lock_guard<std::mutex> lk(reg.mu);
     for (auto& p : reg.layers)
@@ -334,8 +336,8 @@ class BertAttention {
     return r;
   }
 
-  void kick(const std::vector<int32_t>& lens, int device) {
-    drop_plan();
+  void kick(const std::vector<int32_t>& lens, int device, const c10::cuda::CUDAStream& ordered) {
+    check(drop_plan(&ordered));
     if (async_) pending_ = std::async(std::launch::async, &BertAttention::build_plan, this, lens, device);
     else sync_lens_ = lens;
     device_ = device;
@@ -393,9 +395,6 @@ class BertAttention {
     auto pre = info.find("pre_process");
     if (pre != info.end())
       pre->second += std::chrono::duration<float>(std::chrono::steady_clock::now() - t0).count();
-    if (plan_used_ && plan_stream_ != st) plan_shared_ = true;
-    plan_used_ = true;
-    plan_stream_ = st;
     timed(info, "attention", [&] {
       check(rt_sparse_attention(ctx.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), plan_, 1.0f, dtype_, st));
     });
@@ -409,19 +408,16 @@ class BertAttention {
   }
 
  private:
-  void drop_plan() {
+  // Gives the plan back: behind `ordered`, a stream that is behind every use (update_meta_data's, under its
+  // SharedUse), or else after a wait for the plan's device.
+  rt_status drop_plan(const c10::cuda::CUDAStream* ordered) {
+    rt_attn_plan* plan = std::exchange(plan_, nullptr);
     if (pending_.valid()) {
       PlanResult r = pending_.get();
       if (r.plan) rt_attn_plan_destroy(r.plan);
     }
-    if (plan_) {
-      // the previous batch's attention kernel may still read it: its memory is free again behind the stream that
-      // ran it; a plan that several streams used waits for the device
-      if (plan_used_ && !plan_shared_) rt_attn_plan_destroy_on(plan_, plan_stream_);
-      else rt_attn_plan_destroy(plan_);
-      plan_ = nullptr;
-    }
-    plan_used_ = plan_shared_ = false;
+    if (ordered && ordered->device_index() == device_) return rt_attn_plan_destroy_on(plan, ordered->stream());
+    return rt_attn_plan_destroy(plan);
   }
 
   int heads_, hidden_ = 0, layer_idx_, dtype_ = RT_F16, device_ = 0;
@@ -430,8 +426,6 @@ class BertAttention {
   std::future<PlanResult> pending_;
   std::vector<int32_t> sync_lens_;
   rt_attn_plan* plan_ = nullptr;
-  bool plan_used_ = false, plan_shared_ = false;  // the current plan has been launched / from more than one stream
-  void* plan_stream_ = nullptr;
 };
 
 class MetaData {
@@ -470,7 +464,7 @@ class MetaData {
     LayerRegistry::upload(reg.seq_prefix, seq_len_info);
     reg.n_seq = static_cast<int>(lens.size());
     for (BertAttention* l : reg.layers)
-      if (l) l->kick(lens, device);
+      if (l) l->kick(lens, device, use.stream());
   }
   // layers/metadata.cpp:20-27: shutdown; here: join every pending host task
   void terminate_thread() {

@@ -154,3 +154,27 @@ def test_captured_forward_replays():
     assert torch.equal(out, flipped)
     md.terminate_thread()
     ops.check_device()
+
+
+def test_stream_destroyed_between_batches():
+    """Nothing of a batch on a caller's own stream is touched through that stream once the caller has waited for it and
+    destroyed it."""
+    import ctypes
+    from raptor_t_b200 import ops
+    md, batches, update, forward = _model_and_batches(2, [[4096, 512], [832, 1024]])
+    want = _wanted(batches, update, forward)
+    rt = torch.cuda.cudart()
+    for i in range(4):
+        handle = ctypes.c_ulonglong(0)
+        assert int(rt.cudaStreamCreate(ctypes.addressof(handle))) == 0
+        own = torch.cuda.ExternalStream(handle.value)
+        update(batches[i % 2])
+        with torch.cuda.stream(own):
+            out = forward(batches[i % 2])
+        own.synchronize()
+        assert int(rt.cudaStreamDestroy(handle.value)) == 0
+        assert torch.equal(out, want[i % 2])
+    update(batches[1])
+    assert torch.equal(forward(batches[1]), want[1])
+    md.terminate_thread()
+    ops.check_device()
