@@ -72,7 +72,12 @@ struct DevBuf {
     if (p) cudaFree(p);
     p = nullptr;
     bytes = 0;
-    RT_CHECK_CUDA(cudaMalloc(&p, need));
+    const cudaError_t e = cudaMalloc(&p, need);
+    if (e != cudaSuccess) {
+      p = nullptr;
+      cudaGetLastError();  // reported here: the next launch's check must not see it again
+      return fail(RT_ERR_CUDA, "cudaMalloc of %zu bytes failed: %s", need, cudaGetErrorString(e));
+    }
     bytes = need;
     return RT_OK;
   }
@@ -393,6 +398,10 @@ rt_status ensure_scratch(rt_encoder* e, int tokens) {
   const size_t parts = std::min(T * H * 4 * kMaxLnSplits, kLnPartsBytes);
   size_t total = parts;
   for (const auto& n : names) total += align256(n.second);
+  // the old memory goes before the larger one is there: if that fails, nothing may still point at it
+  e->capacity_tokens = 0;
+  e->scratch.clear();
+  e->ln_parts = {};
   RT_TRY(e->scratch_mem.ensure(total));
   uint8_t* at = static_cast<uint8_t*>(e->scratch_mem.p);
   for (const auto& n : names) {
