@@ -20,6 +20,7 @@
 #include <chrono>
 #include <condition_variable>
 #include <cstring>
+#include <initializer_list>
 #include <map>
 #include <mutex>
 #include <string>
@@ -456,6 +457,16 @@ bool fuses_layernorm(const rt_encoder* e, int K) {
   return blocks > 10 && (K < 2048 || blocks <= 15 || blocks > 48);
 }
 
+// The caller's pointers of a projection + LayerNorm.  The cluster kernel takes 32-byte aligned ones; a projection that
+// is fused for speed alone (fuse_layernorm 1, other than the 768-wide FFN down, which has no other path for large
+// batches) falls back to the separate kernels, which take 16.
+bool aligned(size_t bytes, std::initializer_list<const void*> ptrs) {
+  uintptr_t all = 0;
+  for (const void* p : ptrs) all |= reinterpret_cast<uintptr_t>(p);
+  return (all & (bytes - 1)) == 0;
+}
+bool always_fused(const rt_encoder* e, int K) { return e->fuse_layernorm == 2 || (e->cfg.hidden == 768 && K >= 2048); }
+
 rt_status run_parts(rt_encoder* e, const GemmPlan& plan, const char* span, void* out, const void* a, const void* w,
                     const void* bias, const void* residual, const void* gamma, const void* beta, int K, cudaStream_t st) {
   const rt_config& c = e->cfg;
@@ -507,7 +518,7 @@ rt_status run_attention(rt_encoder* e, int l, const void* input, void* output, c
                                    AttnSplit{reinterpret_cast<const int32_t*>(dev + e->groups_off), e->plan_groups[l],
                                              static_cast<float*>(e->part_o.p), static_cast<float*>(e->part_ml.p)}));
   }
-  if (fuses_layernorm(e, H)) {
+  if (fuses_layernorm(e, H) && (always_fused(e, H) || aligned(32, {output, input}))) {
     Span s(e, st, "gemm.attention_output");
     RT_TRY(rt_gemm_bias_residual_layernorm(output, ctx, w.ao_w.p, w.ao_b.p, input, w.aln_g.p, w.aln_b.p, T, H, H, c.eps,
                                            dt, st));
@@ -553,9 +564,13 @@ rt_status run_output(rt_encoder* e, int l, const void* ffn, const void* residual
   RT_REQUIRE(w.set, RT_ERR_STATE, "layer %d has no weights", l);
   void* dense = e->scratch["dense_out"].p;
   GemmPlan parts;
-  if (plan_parts(e, c.ffn, parts))
+  if (plan_parts(e, c.ffn, parts)) {
+    // no kernel behind this checks them: as the paths of larger batches require
+    const int bytes = always_fused(e, c.ffn) ? 32 : 16;
+    RT_REQUIRE(aligned(bytes, {ffn, residual, out}), RT_ERR_INVALID, "output: pointers must be %d-byte aligned", bytes);
     return run_parts(e, parts, "gemm.ffn_down", out, ffn, w.down_w.p, w.down_b.p, residual, w.oln_g.p, w.oln_b.p, c.ffn, st);
-  if (fuses_layernorm(e, c.ffn)) {
+  }
+  if (fuses_layernorm(e, c.ffn) && (always_fused(e, c.ffn) || aligned(32, {ffn, residual, out}))) {
     Span s(e, st, "gemm.ffn_down");
     return rt_gemm_bias_residual_layernorm(out, ffn, w.down_w.p, w.down_b.p, residual, w.oln_g.p, w.oln_b.p, e->tokens,
                                            c.hidden, c.ffn, c.eps, c.dtype, st);
