@@ -204,10 +204,10 @@ __global__ void __launch_bounds__(1024) layernorm_parts_kernel(T* __restrict__ o
   const size_t at = static_cast<size_t>(blockIdx.x) * hidden + col;
   const float inv_h = 1.0f / static_cast<float>(hidden);
   float bb[4], gg[4], be[4], rr[4], v[4] = {0.f, 0.f, 0.f, 0.f};
+  RT_PDL_WAIT();
   unpack4(bias + col, bb);
   unpack4(gamma + col, gg);
   unpack4(beta + col, be);
-  RT_PDL_WAIT();
   unpack4(residual + at, rr);
   const size_t stride = static_cast<size_t>(rows) * hidden;
 #pragma unroll 4

@@ -191,10 +191,6 @@ gemm_ln_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     *cta_abort = 0;
     fence_barrier_init();
   }
-  for (int i = threadIdx.x; i < 3 * TW / 2; i += kThreads) {
-    const uint16_t* src = i < TW / 2 ? bias : i < TW ? gamma : beta;
-    reinterpret_cast<float2*>(params)[i] = unpack2<BF16>(reinterpret_cast<const uint32_t*>(src + tile * TW)[i % (TW / 2)]);
-  }
   if (warp == 1) {
     if constexpr (PAIR) {
       tmem_alloc_pair(tmem_slot, kTmemCols);
@@ -209,7 +205,7 @@ gemm_ln_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   cluster_arrive();  // every peer's barriers exist before anything remote touches them
   cluster_wait();
   tc_fence_after_sync();
-  RT_PDL_WAIT();  // operands, residual and the output buffer belong to the previous kernel until here
+  RT_PDL_WAIT();  // operands, parameters, residual and the output buffer belong to the previous kernel until here
   const uint32_t tmem_base = *tmem_slot;
   AbortCtx ab{cta_abort, error_flag};
 
@@ -311,6 +307,11 @@ gemm_ln_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     uint32_t tile_it = 0, res_phase = 0;
     bool ok = true;
     if (cluster_id < n_tiles_m) load_residual(cluster_id, set);
+    for (int i = threadIdx.x - 128; i < 3 * TW / 2; i += kEpilogueThreads) {  // under the first main loop
+      const uint16_t* src = i < TW / 2 ? bias : i < TW ? gamma : beta;
+      reinterpret_cast<float2*>(params)[i] = unpack2<BF16>(reinterpret_cast<const uint32_t*>(src + tile * TW)[i % (TW / 2)]);
+    }
+    asm volatile("bar.sync 1, %0;" ::"n"(kEpilogueThreads) : "memory");
     for (int t = cluster_id; t < n_tiles_m && ok; t += n_clusters, ++tile_it) {
       const int a = tile_it & 1;
       const uint32_t aph = (tile_it >> 1) & 1;
