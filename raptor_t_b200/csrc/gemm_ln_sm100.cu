@@ -8,8 +8,8 @@
 // columns [256 p, 256 p + 256) with the same cta_group::2 main loop as gemm_pair_sm100.cu, and
 // the epilogue
 //   1. reads the fp32 accumulator into registers once, adds bias and residual there (never rounded to 16 bits), and
-//      sums x and x^2 over the thread's columns,
-//   2. sends those partial sums to every CTA of the cluster that holds the same rows (distributed shared memory:
+//      forms the sum and the squared deviations of the thread's columns,
+//   2. sends both to every CTA of the cluster that holds the same rows (distributed shared memory:
 //      st.async, whose bytes the receiver's mbarrier counts),
 //   3. waits for all partials of its rows, forms mean and 1/sigma, normalises its columns and
 //      stores the 16-bit result.
@@ -52,7 +52,7 @@ constexpr int kRegsIssue = 72;
 constexpr int kRegsEpilogue = 216;
 constexpr int kTmemCols = 512;          // two 256-column accumulators
 constexpr int kMaxNT = 4;               // N up to 1024
-// row statistics: [accumulator parity][partial slot = n-tile * 2 + column-parity warp][row of this CTA] {sum, sum of squares}
+// row statistics: [accumulator parity][partial slot = n-tile * 2 + column-parity warp][row of this CTA] {sum, squared deviations from the part's mean}
 constexpr int kStatsBytes = 2 * (2 * kMaxNT) * 128 * 8;
 constexpr int kBoxBytes = 32 * 64 * 2;  // residual / result box of one epilogue warp
 // Shape of a cluster: NT column tiles of TW columns, each computed by a CTA pair (256 rows) or by one CTA (128 rows).
@@ -289,6 +289,7 @@ gemm_ln_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     const int quarter = warp & 3;        // TMEM lane quarter
     const int set = (warp - 4) >> 2;     // this warp takes the 64-column boxes set, set + 2 of its 32 rows
     constexpr int kBoxes = TW / 64;
+    const bool two_boxes = set + 2 < kBoxes;
     const int row_local = quarter * 32 + lane;
     const uint32_t leader_acc_empty[2] = {map_to_rank(&acc_empty[0], leader), map_to_rank(&acc_empty[1], leader)};
     const int n0 = tile * TW;
@@ -318,8 +319,8 @@ gemm_ln_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       if (!mbar_wait(&acc_full[a], aph, ab, 124)) { ok = false; break; }
       tc_fence_after_sync();
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + a * kTileN;
-      // pass 1: x = acc + bias + residual in registers; partial sums of x and x^2
-      uint64_t sum2 = 0, sq2 = 0;  // packed pairs of fp32
+      // pass 1: x = acc + bias + residual in registers; sum of x over the thread's columns
+      uint64_t sum2 = 0;  // packed pair of fp32
       uint32_t x[128];
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
@@ -343,7 +344,6 @@ gemm_ln_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
               uint32_t* v = x + i * 64 + q * 8 + 2 * j;
               const uint64_t y = f2_add(f2_add(f2_pack(__uint_as_float(v[0]), __uint_as_float(v[1])), bb[j]), f2_pack(rr.x, rr.y));
               sum2 = f2_add(sum2, y);
-              sq2 = f2_fma(y, y, sq2);
               const float2 f = f2_unpack(y);
               v[0] = __float_as_uint(f.x);
               v[1] = __float_as_uint(f.y);
@@ -355,29 +355,53 @@ gemm_ln_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           }
         }
       }
-      const float2 sums = f2_unpack(sum2), sqs = f2_unpack(sq2);
-      const float sum = sums.x + sums.y, sq = sqs.x + sqs.y;
+      const float2 sums = f2_unpack(sum2);
+      const float sum = sums.x + sums.y;
       // the accumulator is in registers: the tile after the next may overwrite it
       tc_fence_before_sync();
       mbar_arrive_cluster(leader_acc_empty[a]);
       if (!ok) break;
+      // squared deviations from the mean of the thread's own columns: no cancellation, however far the row's mean is
+      // above its deviation
+      const float own_mean = sum * (1.0f / 64) * (two_boxes ? 0.5f : 1.0f);
+      const uint64_t neg_own = f2_pack(-own_mean, -own_mean);
+      uint64_t dev2[2] = {0, 0};
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        if (set + 2 * i < kBoxes) {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) {
+            const uint32_t* v = x + i * 64 + 2 * j;
+            const uint64_t d = f2_add(f2_pack(__uint_as_float(v[0]), __uint_as_float(v[1])), neg_own);
+            dev2[j & 1] = f2_fma(d, d, dev2[j & 1]);
+          }
+        }
+      }
+      const float2 devs = f2_unpack(f2_add(dev2[0], dev2[1]));
+      const float dev = devs.x + devs.y;
       // the partial sums go to every CTA that holds these rows (same hrow, every column tile); a peer cannot be two
       // tiles ahead (its wait for the tile between needs this CTA's sums), so the barrier is in this tile's phase
       if (warp == 4 && lane == 0) mbar_arrive_expect_tx(&stats_full[a], NT * kEpilogueThreads * 8);
 #pragma unroll
       for (int p = 0; p < NT; ++p)
-        st_async_f2(map_to_rank(stats + (a * (2 * kMaxNT) + slot) * 128 + row_local, peer_of(p)), sum, sq,
+        st_async_f2(map_to_rank(stats + (a * (2 * kMaxNT) + slot) * 128 + row_local, peer_of(p)), sum, dev,
                     map_to_rank(&stats_full[a], peer_of(p)));
       if (!mbar_wait_cluster(&stats_full[a], aph, ab, 125)) { ok = false; break; }
-      float tot = 0.f, tot_sq = 0.f;
+      float2 part[kSlots];
+      float tot = 0.f, tot_dev = 0.f;
 #pragma unroll
       for (int sl = 0; sl < kSlots; ++sl) {
-        const float2 v = stats[(a * (2 * kMaxNT) + sl) * 128 + row_local];
-        tot += v.x;
-        tot_sq += v.y;
+        part[sl] = stats[(a * (2 * kMaxNT) + sl) * 128 + row_local];
+        tot += part[sl].x;
       }
       const float mean = tot * (1.0f / N);
-      const float var = fmaxf(tot_sq * (1.0f / N) - mean * mean, 0.f);
+#pragma unroll
+      for (int sl = 0; sl < kSlots; ++sl) {  // deviations about the part's mean -> about the row's
+        const int cols = 64 * ((kBoxes + 1 - (sl & 1)) / 2);  // of the warps of this set
+        const float d = part[sl].x * (1.0f / cols) - mean;
+        tot_dev += fmaf(d * d, static_cast<float>(cols), part[sl].y);
+      }
+      const float var = tot_dev * (1.0f / N);
       const float rstd = rsqrtf(var + eps);
       // pass 2: normalise this thread's columns, store them box by box
       const int row0 = row0_of(t);
