@@ -54,6 +54,7 @@ constexpr int kTmemCols = 512;          // two 256-column accumulators
 constexpr int kMaxNT = 4;               // N up to 1024
 // row statistics: [accumulator parity][partial slot = n-tile * 2 + column-parity warp][row of this CTA] {sum, squared deviations from the part's mean}
 constexpr int kStatsBytes = 2 * (2 * kMaxNT) * 128 * 8;
+constexpr int kDrainTries = 1 << 16;    // each suspends the thread for some time
 constexpr int kBoxBytes = 32 * 64 * 2;  // residual / result box of one epilogue warp
 // Shape of a cluster: NT column tiles of TW columns, each computed by a CTA pair (256 rows) or by one CTA (128 rows).
 template <bool PAIR, int NT, int TW>
@@ -298,8 +299,10 @@ gemm_ln_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     uint8_t* const line = box + lane * 128;
     const int swz = lane & 7;
     uint64_t* const my_res = &res_full[warp - 4];
+    bool res_on_its_way = false;
     auto row0_of = [&](int t) { return t * Cfg::kRows + static_cast<int>(hrow) * 128 + quarter * 32; };
     auto load_residual = [&](int t, int b) {
+      res_on_its_way = true;
       if (lane == 0) {
         mbar_arrive_expect_tx(my_res, kBoxBytes);
         tma_load_2d(box, &map_res, n0 + b * 64, row0_of(t), my_res);
@@ -329,7 +332,8 @@ gemm_ln_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           tmem_ld32(taddr + b * 64, x + i * 64);
           tmem_ld32(taddr + b * 64 + 32, x + i * 64 + 32);
           if (!mbar_wait(my_res, res_phase, ab, 126)) ok = false;
-          res_phase ^= 1;
+          else res_on_its_way = false;
+          res_phase ^= ok;
           tc_wait_ld();
 #pragma unroll
           for (int q = 0; q < 8; ++q) {
@@ -351,7 +355,7 @@ gemm_ln_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           }
           if (i == 0 && set + 2 < kBoxes) {
             __syncwarp();  // every lane has read its line
-            load_residual(t, set + 2);
+            if (ok) load_residual(t, set + 2);
           }
         }
       }
@@ -444,6 +448,8 @@ gemm_ln_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         load_residual(t + n_clusters, set);
       }
     }
+    // left early (a wait ran out): the CTA must not end under a box that is still on its way to it
+    for (int i = 0; res_on_its_way && i < kDrainTries; ++i) res_on_its_way = !mbar_try_wait(my_res, res_phase);
     if (lane == 0) tma_store_wait<0>();  // the boxes are read and the result written before the CTA ends
   }
 
