@@ -717,19 +717,25 @@ rt_status launch_sparse_attention(void* ctx, const void* q, const void* k, const
 using namespace rt;
 
 namespace {
-// Device memory of plans: a pool per device that keeps up to kPlanPoolBytes of freed memory.  A serving loop
+// Device memory of plans: a pool per device that keeps up to kPlanPoolBytes of freed memory while there are plans, and
+// gives it back with the last one that is destroyed.  A serving loop
 // that builds a plan per layer and batch would otherwise spend its time in cudaMalloc / cudaFree of a few MB
 // (0.5 ms and 0.27 ms each, more with several threads, against 50 us for everything else of an upload).
 constexpr uint64_t kPlanPoolBytes = 64u << 20;
 
-rt_status plan_pool(cudaMemPool_t* out) {
-  static std::mutex mu;
-  static cudaMemPool_t pools[64] = {};
-  int dev = 0;
-  RT_CHECK_CUDA(cudaGetDevice(&dev));
+struct PlanPool {
+  std::mutex mu;
+  cudaMemPool_t pool = nullptr;
+  int plans = 0;  // that hold memory of it
+};
+PlanPool plan_pools[64];
+
+// One more plan is about to take memory of the current device's pool.
+rt_status plan_pool(int dev, cudaMemPool_t* out) {
   RT_REQUIRE(dev >= 0 && dev < 64, RT_ERR_UNSUPPORTED, "device index %d out of range", dev);
-  std::lock_guard<std::mutex> lk(mu);
-  if (!pools[dev]) {
+  PlanPool& p = plan_pools[dev];
+  std::lock_guard<std::mutex> lk(p.mu);
+  if (!p.pool) {
     cudaMemPoolProps props{};
     props.allocType = cudaMemAllocationTypePinned;
     props.location.type = cudaMemLocationTypeDevice;
@@ -740,10 +746,18 @@ rt_status plan_pool(cudaMemPool_t* out) {
     int no = 0;  // a new plan takes memory that is already free or fresh memory, it never waits for a kernel
     cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
     cudaMemPoolSetAttribute(pool, cudaMemPoolReuseAllowInternalDependencies, &no);
-    pools[dev] = pool;
+    p.pool = pool;
   }
-  *out = pools[dev];
+  ++p.plans;
+  *out = p.pool;
   return RT_OK;
+}
+
+// A plan holds no memory any more; trim: the device has been waited for, so what the last plan leaves can go.
+void plan_gone(int dev, bool trim) {
+  PlanPool& p = plan_pools[dev];
+  std::lock_guard<std::mutex> lk(p.mu);
+  if (--p.plans == 0 && trim) cudaMemPoolTrimTo(p.pool, 0);
 }
 }  // namespace
 
@@ -790,7 +804,7 @@ extern "C" rt_status rt_attn_plan_create(const rt_config* cfg, const int32_t* le
   p->bytes = p->part_ml_off + align(static_cast<size_t>(p->host.n_slots) * 128 * 2 * sizeof(float)) + 256;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   cudaMemPool_t pool = nullptr;
-  s = plan_pool(&pool);
+  s = plan_pool(p->device, &pool);
   if (s != RT_OK) {
     delete p;
     return s;
@@ -811,6 +825,7 @@ extern "C" rt_status rt_attn_plan_create(const rt_config* cfg, const int32_t* le
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) {
     if (p->dev) cudaFreeAsync(p->dev, st);
+    plan_gone(p->device, false);
     delete p;
     return fail(RT_ERR_CUDA, "attn_plan_create: %s", cudaGetErrorString(e));
   }
@@ -841,6 +856,7 @@ extern "C" rt_status rt_attn_plan_destroy(rt_attn_plan* p) {
     e = on.status;
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
     if (e == cudaSuccess) e = cudaFree(p->dev);
+    if (e == cudaSuccess) plan_gone(p->device, true);
   }
   delete p;
   if (e != cudaSuccess) return fail(RT_ERR_CUDA, "attn_plan_destroy: %s", cudaGetErrorString(e));
@@ -855,6 +871,7 @@ extern "C" rt_status rt_attn_plan_destroy_on(rt_attn_plan* p, void* stream) {
       cudaGetLastError();  // handled: the next launch must not report it
       return rt_attn_plan_destroy(p);
     }
+    plan_gone(p->device, false);
   }
   delete p;
   return RT_OK;
