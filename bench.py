@@ -348,6 +348,7 @@ def run_gpu(args, w):
     stage_flops = [0.0, 0.0]
     stage_tokens = 0
     ln_in_ao, ln_in_down = enc.layernorm_in_projection()
+    parts = enc.get_option("ffn_down_parts")
     for i in range(args.steps):
         flush.fill_(1)
         b = step()
@@ -449,7 +450,9 @@ def run_gpu(args, w):
     fused_ms = sum(stage_ms.get(k, 0.0) for k in fused_keys)
     fused_tf = sum(fl[k] for k in fused_keys) / (fused_ms * 1e-3) / 1e12 if fused_ms else 0.0
     ln_launches = L * (2 - len(fused_keys))
-    ln_gbs = (ln_launches * 3 * stage_tokens * H * 2) / (ln_ms * 1e-3) / 1e9 if ln_ms else 0.0
+    # 16-bit projection and residual in, result out; a split-K FFN down leaves fp32 parts in place of the projection
+    ln_bytes = L * ((not ln_in_ao) * 6 + (4 * parts + 4 if parts else (not ln_in_down) * 6)) * stage_tokens * H
+    ln_gbs = ln_bytes / (ln_ms * 1e-3) / 1e9 if ln_ms else 0.0
     tr_gbs = (L * 2 * stage_tokens * 3 * H * 2) / (tr_ms * 1e-3) / 1e9 if tr_ms else 0.0
     if gemm_ms >= attn_ms:
         roof = {"kernel": f"gemm_pair_kernel (CTA-pair tcgen05 projection GEMMs: {', '.join(k[5:] for k in pair_keys)})",

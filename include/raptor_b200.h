@@ -306,7 +306,8 @@ rt_status rt_encoder_kernel_launches(rt_encoder* enc, int64_t* launches_out);
  * "fuse_residual" (1: bias + residual added in the projection GEMM's epilogue, LayerNorm reads one tensor;
  * default 0: it costs one more 16-bit rounding and measured slower; ignored where fuse_layernorm applies).
  * fuse_gelu, fuse_qkv and fuse_layernorm default to 1.  rt_encoder_get_option also answers
- * "layernorm_in_attention_output" and "layernorm_in_ffn_down": what the prepared batch does. */
+ * "layernorm_in_attention_output", "layernorm_in_ffn_down" and "ffn_down_parts" (fp32 parts of a split-K FFN down,
+ * 0: not split): what the prepared batch does. */
 rt_status rt_encoder_set_option(rt_encoder* enc, const char* name, int value);
 rt_status rt_encoder_get_option(rt_encoder* enc, const char* name, int* value_out);
 /* work-list statistics of one layer of the prepared batch */

@@ -774,9 +774,11 @@ extern "C" rt_status rt_encoder_get_option(rt_encoder* e, const char* name, int*
   else if (std::strcmp(name, "fuse_layernorm") == 0) *value_out = e->fuse_layernorm;
   else if (std::strcmp(name, "fuse_residual") == 0) *value_out = e->fuse_residual;
   else if (std::strcmp(name, "layernorm_in_attention_output") == 0) *value_out = fuses_layernorm(e, e->cfg.hidden);
-  else if (std::strcmp(name, "layernorm_in_ffn_down") == 0) {
-    GemmPlan parts;
-    *value_out = !plan_parts(e, e->cfg.ffn, parts) && fuses_layernorm(e, e->cfg.ffn);
+  else if (std::strcmp(name, "layernorm_in_ffn_down") == 0 || std::strcmp(name, "ffn_down_parts") == 0) {
+    GemmPlan plan;
+    const bool parts = plan_parts(e, e->cfg.ffn, plan);
+    if (name[0] == 'f') *value_out = parts ? plan.splits : 0;
+    else *value_out = !parts && fuses_layernorm(e, e->cfg.ffn);
   } else return fail(RT_ERR_INVALID, "get_option: unknown option '%s'", name);
   return RT_OK;
 }
