@@ -144,9 +144,9 @@ rt_status rt_gemm_residual(void* c_dev, const void* a_dev, const void* w_dev, co
 
 /* out[M][N] = LayerNorm(A W^T + bias + residual) * gamma + beta in ONE kernel, N = 768 or 1024: the
  * projection and the add_bias_and_layernorm kernel that follows it in both sub-layers
- * (layers/multi_headed_attention.cpp:206-210, layers/bert_output.cpp:19-23).  A cluster of N/256 CTA
- * pairs owns 256 whole rows; the pre-LayerNorm sum stays in fp32 in TMEM and never reaches HBM.
- * All pointers 32-byte aligned, K % 64 == 0; out may alias residual. */
+ * (layers/multi_headed_attention.cpp:206-210, layers/bert_output.cpp:19-23).  A cluster owns whole rows:
+ * N/256 CTA pairs 256 of them, or (N = 768, few rows) four single CTAs 128; the pre-LayerNorm sum stays in
+ * fp32 registers and never reaches HBM.  All pointers 32-byte aligned, K % 64 == 0; out may alias residual. */
 rt_status rt_gemm_bias_residual_layernorm(void* out_dev, const void* a_dev, const void* w_dev, const void* bias_dev,
                                           const void* residual_dev, const void* gamma_dev, const void* beta_dev,
                                           int M, int N, int K, float eps, int dtype, void* stream);
@@ -300,9 +300,10 @@ rt_status rt_encoder_enable_timing(rt_encoder* enc, int on);
 rt_status rt_encoder_kernel_launches(rt_encoder* enc, int64_t* launches_out);
 /* options: "fuse_gelu" (1: bias+GELU in the FFN-up GEMM epilogue, 0: separate rt_bias_gelu kernel);
  * "fuse_qkv" (1: rt_gemm_qkv, 0: rt_gemm + rt_qkv_bias_transpose); "fuse_layernorm" (LayerNorm in the epilogue of
- * the hidden-wide projections of 768- and 1024-wide models, rt_gemm_bias_residual_layernorm: 0 never; 1 where it
- * measured faster for the batch's token count, small batches take a split-K GEMM whose fp32 parts LayerNorm sums;
- * 2 always);
+ * the hidden-wide projections of 768- and 1024-wide models, rt_gemm_bias_residual_layernorm: 0 never; 1 by the
+ * batch's token count, from measured times, small batches take a split-K GEMM whose fp32 parts LayerNorm sums;
+ * 2 always; with 1 or 2 the last bits of a sequence's result depend on the tokens it is batched with, with 0
+ * only through cuts of long attention lists);
  * "fuse_residual" (1: bias + residual added in the projection GEMM's epilogue, LayerNorm reads one tensor;
  * default 0: it costs one more 16-bit rounding and measured slower; ignored where fuse_layernorm applies).
  * fuse_gelu, fuse_qkv and fuse_layernorm default to 1.  rt_encoder_get_option also answers

@@ -15,7 +15,8 @@
 //      stores the 16-bit result.
 // Residual and result travel as 32-row x 64-column TMA boxes through 4 KB of shared memory per epilogue warp, bias,
 // gamma and beta sit in shared memory.  The epilogue is a chain of latencies (SM clocks per tile, 20480 rows: pass 1
-// 4300, exchange 4200, pass 2 3500) and outlasts a K = 768 main loop; one under K = 3072 is hidden.  Against
+// 4300, exchange 1550-1800, pass 2 3500, the passes before their packed-pair arithmetic) and outlasts a K = 768 main
+// loop; one under K = 3072 is hidden.  Against
 // row-wise loads and stores by the threads and a second pass over TMEM: K = 3072, 8192 rows 40.2 -> 36.8 us.
 // The pre-LayerNorm sum therefore never reaches HBM, the separate LayerNorm launch disappears,
 // and one 16-bit rounding per sub-layer with it.  No TMA multicast is used anywhere.
@@ -52,7 +53,8 @@ constexpr int kRegsIssue = 72;
 constexpr int kRegsEpilogue = 216;
 constexpr int kTmemCols = 512;          // two 256-column accumulators
 constexpr int kMaxNT = 4;               // N up to 1024
-// row statistics: [accumulator parity][partial slot = n-tile * 2 + column-parity warp][row of this CTA] {sum, squared deviations from the part's mean}
+// row statistics: [accumulator parity][partial slot = n-tile * 2 + column-parity warp][row of this CTA]
+// {sum, squared deviations from the part's mean}
 constexpr int kStatsBytes = 2 * (2 * kMaxNT) * 128 * 8;
 constexpr int kDrainTries = 1 << 16;    // each suspends the thread for some time
 constexpr int kBoxBytes = 32 * 64 * 2;  // residual / result box of one epilogue warp
