@@ -8,7 +8,7 @@
 // columns [256 p, 256 p + 256) with the same cta_group::2 main loop as gemm_pair_sm100.cu, and
 // the epilogue
 //   1. reads the fp32 accumulator into registers once, adds bias and residual there (never rounded to 16 bits), and
-//      forms the sum and the squared deviations of the thread's columns,
+//      forms the mean and the squared deviations of the thread's columns,
 //   2. sends both to every CTA of the cluster that holds the same rows (distributed shared memory:
 //      st.async, whose bytes the receiver's mbarrier counts),
 //   3. waits for all partials of its rows, forms mean and 1/sigma, normalises its columns and
@@ -54,7 +54,7 @@ constexpr int kRegsEpilogue = 216;
 constexpr int kTmemCols = 512;          // two 256-column accumulators
 constexpr int kMaxNT = 4;               // N up to 1024
 // row statistics: [accumulator parity][partial slot = n-tile * 2 + column-parity warp][row of this CTA]
-// {sum, squared deviations from the part's mean}
+// {mean, squared deviations from it}
 constexpr int kStatsBytes = 2 * (2 * kMaxNT) * 128 * 8;
 constexpr int kDrainTries = 1 << 16;    // each suspends the thread for some time
 constexpr int kBoxBytes = 32 * 64 * 2;  // residual / result box of one epilogue warp
@@ -324,8 +324,13 @@ gemm_ln_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       if (!mbar_wait(&acc_full[a], aph, ab, 124)) { ok = false; break; }
       tc_fence_after_sync();
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + a * kTileN;
-      // pass 1: x = acc + bias + residual in registers; sum of x over the thread's columns
-      uint64_t sum2 = 0;  // packed pair of fp32
+      // pass 1: x = acc + bias + residual, kept in registers as its distance d from the mean of the thread's first eight
+      // columns; sums of d and d^2 over all of them.  That mean is within sqrt(15) deviations of the mean of the
+      // thread's 128, whatever the values are, so that sum d^2 - (sum d)^2 / n costs four bits at most, where
+      // E[x^2] - mean^2 costs all that a row's mean is above its deviation.  Against that form, 768 columns: 20480 rows
+      // K = 768 32.1 -> 33.0 us, K = 3072 80.2 -> 80.8; 5312 rows 22.9 -> 23.0.
+      uint64_t sum2 = 0, sq2 = 0, neg_shift = 0;  // packed pairs of fp32
+      float shift = 0.f;
       uint32_t x[128];
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
@@ -344,13 +349,25 @@ gemm_ln_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             const ulonglong2 b01 = bv[0], b23 = bv[1];
             const uint64_t bb[4] = {b01.x, b01.y, b23.x, b23.y};
             const uint32_t rw[4] = {r4.x, r4.y, r4.z, r4.w};
+            uint64_t y[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
               const float2 rr = unpack2<BF16>(rw[j]);
+              const uint32_t* v = x + i * 64 + q * 8 + 2 * j;
+              y[j] = f2_add(f2_add(f2_pack(__uint_as_float(v[0]), __uint_as_float(v[1])), bb[j]), f2_pack(rr.x, rr.y));
+            }
+            if (i == 0 && q == 0) {
+              const float2 first = f2_unpack(f2_add(f2_add(y[0], y[1]), f2_add(y[2], y[3])));
+              shift = (first.x + first.y) * 0.125f;
+              neg_shift = f2_pack(-shift, -shift);
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const uint64_t d = f2_add(y[j], neg_shift);
+              sum2 = f2_add(sum2, d);
+              sq2 = f2_fma(d, d, sq2);
+              const float2 f = f2_unpack(d);
               uint32_t* v = x + i * 64 + q * 8 + 2 * j;
-              const uint64_t y = f2_add(f2_add(f2_pack(__uint_as_float(v[0]), __uint_as_float(v[1])), bb[j]), f2_pack(rr.x, rr.y));
-              sum2 = f2_add(sum2, y);
-              const float2 f = f2_unpack(y);
               v[0] = __float_as_uint(f.x);
               v[1] = __float_as_uint(f.y);
             }
@@ -361,57 +378,39 @@ gemm_ln_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           }
         }
       }
-      const float2 sums = f2_unpack(sum2);
-      const float sum = sums.x + sums.y;
+      const float2 sums = f2_unpack(sum2), sqs = f2_unpack(sq2);
+      const float sum = sums.x + sums.y, own = sum * (two_boxes ? 1.0f / 128 : 1.0f / 64);
+      const float own_mean = shift + own, dev = fmaxf(fmaf(-sum, own, sqs.x + sqs.y), 0.f);
       // the accumulator is in registers: the tile after the next may overwrite it
       tc_fence_before_sync();
       mbar_arrive_cluster(leader_acc_empty[a]);
       if (!ok) break;
-      // squared deviations from the mean of the thread's own columns: no cancellation, however far the row's mean is
-      // above its deviation
-      const float own_mean = sum * (1.0f / 64) * (two_boxes ? 0.5f : 1.0f);
-      const uint64_t neg_own = f2_pack(-own_mean, -own_mean);
-      uint64_t dev2[2] = {0, 0};
-#pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        if (set + 2 * i < kBoxes) {
-#pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            const uint32_t* v = x + i * 64 + 2 * j;
-            const uint64_t d = f2_add(f2_pack(__uint_as_float(v[0]), __uint_as_float(v[1])), neg_own);
-            dev2[j & 1] = f2_fma(d, d, dev2[j & 1]);
-          }
-        }
-      }
-      const float2 devs = f2_unpack(f2_add(dev2[0], dev2[1]));
-      const float dev = devs.x + devs.y;
-      // the partial sums go to every CTA that holds these rows (same hrow, every column tile); a peer cannot be two
-      // tiles ahead (its wait for the tile between needs this CTA's sums), so the barrier is in this tile's phase
+      // mean and deviations go to every CTA that holds these rows (same hrow, every column tile); a peer cannot be two
+      // tiles ahead (its wait for the tile between needs this CTA's), so the barrier is in this tile's phase
       if (warp == 4 && lane == 0) mbar_arrive_expect_tx(&stats_full[a], NT * kEpilogueThreads * 8);
 #pragma unroll
       for (int p = 0; p < NT; ++p)
-        st_async_f2(map_to_rank(stats + (a * (2 * kMaxNT) + slot) * 128 + row_local, peer_of(p)), sum, dev,
+        st_async_f2(map_to_rank(stats + (a * (2 * kMaxNT) + slot) * 128 + row_local, peer_of(p)), own_mean, dev,
                     map_to_rank(&stats_full[a], peer_of(p)));
       if (!mbar_wait_cluster(&stats_full[a], aph, ab, 125)) { ok = false; break; }
       float2 part[kSlots];
-      float tot = 0.f, tot_dev = 0.f;
+      float mean = 0.f, tot_dev = 0.f;
+      auto cols = [](int sl) { return 64 * ((kBoxes + 1 - (sl & 1)) / 2); };  // of the warps of this set
 #pragma unroll
       for (int sl = 0; sl < kSlots; ++sl) {
         part[sl] = stats[(a * (2 * kMaxNT) + sl) * 128 + row_local];
-        tot += part[sl].x;
+        mean = fmaf(part[sl].x, static_cast<float>(cols(sl)) / N, mean);
       }
-      const float mean = tot * (1.0f / N);
 #pragma unroll
       for (int sl = 0; sl < kSlots; ++sl) {  // deviations about the part's mean -> about the row's
-        const int cols = 64 * ((kBoxes + 1 - (sl & 1)) / 2);  // of the warps of this set
-        const float d = part[sl].x * (1.0f / cols) - mean;
-        tot_dev += fmaf(d * d, static_cast<float>(cols), part[sl].y);
+        const float d = part[sl].x - mean;
+        tot_dev += fmaf(d * d, static_cast<float>(cols(sl)), part[sl].y);
       }
       const float var = tot_dev * (1.0f / N);
       const float rstd = rsqrtf(var + eps);
       // pass 2: normalise this thread's columns, store them box by box
       const int row0 = row0_of(t);
-      const uint64_t neg_mean = f2_pack(-mean, -mean), rstd2 = f2_pack(rstd, rstd);
+      const uint64_t to_mean = f2_pack(shift - mean, shift - mean), rstd2 = f2_pack(rstd, rstd);
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
         const int b = set + 2 * i;
@@ -430,7 +429,7 @@ gemm_ln_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
               const uint32_t* v = x + i * 64 + q * 8 + 2 * j;
-              const uint64_t y = f2_mul(f2_add(f2_pack(__uint_as_float(v[0]), __uint_as_float(v[1])), neg_mean), rstd2);
+              const uint64_t y = f2_mul(f2_add(f2_pack(__uint_as_float(v[0]), __uint_as_float(v[1])), to_mean), rstd2);
               const float2 f = f2_unpack(f2_fma(y, gg[j], ee[j]));
               o[j] = pack2<BF16>(f.x, f.y);
             }
