@@ -13,8 +13,7 @@ from raptor_t_b200 import capi, metadata, ops
 cfg = capi.make_config(hidden=768, heads=12, ffn=3072, layers=1, max_pos=16384, vocab=97)
 lens = [16384]
 ptr, idx = metadata.build_block_csr(cfg, 0, lens)
-warm = ops.AttentionPlan(cfg, [1024], *metadata.build_block_csr(cfg, 0, [1024]))
-warm.close()
+torch.zeros(1, device="cuda")
 torch.cuda.synchronize()
 before = torch.cuda.mem_get_info()[0]
 plans = [ops.AttentionPlan(cfg, lens, ptr, idx) for _ in range(6)]
