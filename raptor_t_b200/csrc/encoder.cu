@@ -416,9 +416,10 @@ rt_status ensure_scratch(rt_encoder* e, int tokens) {
 
 // FFN down + LayerNorm for batches of few tokens: split-K GEMM into fp32 parts and a LayerNorm that sums them.
 // The cluster kernel walks all K blocks of a row block in sequence, however few row blocks there are (K = 3072:
-// 17.3 us for 128 rows, 18.2 for 2048, 20.2 for 4096); cut along K until the chip is full, projection and LayerNorm
-// take 8.3 us for 128 rows, 11.7 for 1024, 16.9 for 2048 and 25.1 for 4096.  Estimates in microseconds, as in
-// plan_gemm.  With K = 768 or 1024 the parts' traffic eats the gain (8.0 against 6.9 us for 128 rows): not used.
+// 17.1 us for 128 rows, 17.4 for 1024, 17.9 for 2048, 19.1 for 4096); cut along K until the chip is full, projection
+// and LayerNorm take 9.2 us for 128 rows, 12.3 for 1024, 17.6 for 2048.  Estimates in microseconds, as in plan_gemm
+// (both sides a little high: the line between them lies at 2048 rows).  With K = 768 or 1024 the parts' traffic eats
+// the gain (8.0 against 6.9 us for 128 rows): not used.
 bool plan_parts(const rt_encoder* e, int K, GemmPlan& plan) {
   const int M = e->tokens, N = e->cfg.hidden;
   if (M == 0 || e->fuse_layernorm != 1 || e->fuse_residual || K < 2048 || N % 128 != 0 || N > 4096) return false;
