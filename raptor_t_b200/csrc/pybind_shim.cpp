@@ -19,10 +19,11 @@
 // Every body is a sequence of calls into include/raptor_b200.h; torch is used for the tensors'
 // memory and for the current stream only.  Weights arrive [in, out] (python/modeling_bert.py:
 // 84-91, 107-113, 138-163) and are re-laid-out once to [out, in] for the TMA-fed GEMMs.
-// As in the reference, MetaData::update_meta_data starts one host task per registered
-// attention layer (layers/multi_headed_attention.h:72-110) that builds that layer's block table
-// and work list and uploads them on a side stream while the main thread issues the QKV GEMM;
-// the layer joins its task right before the attention kernel ("pre_process" in info).
+// As in the reference, MetaData::update_meta_data starts host tasks for the registered
+// attention layers (layers/multi_headed_attention.h:72-110) that build a layer's block table
+// and work list and upload them on a side stream while the main thread issues the QKV GEMM;
+// the layer joins its task right before the attention kernel ("pre_process" in info).  Layers
+// whose block lists are the same (BatchPlan) share one task and one work list.
 // The partition tensors and block_limit are accepted for signature compatibility: the kernel's
 // own work list (pairs of query blocks per CTA) is built from the block table.
 #include <torch/extension.h>
@@ -31,9 +32,11 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 
+#include <array>
 #include <chrono>
 #include <future>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <optional>
 #include <stdexcept>
@@ -293,6 +296,75 @@ struct PlanResult {
   std::string error;
 };
 
+// Block table of one layer (seeded by its index) -> work list -> upload.
+PlanResult build_plan(const rt_config& c, uint32_t seed, const std::vector<int32_t>& lens, int device) {
+  PlanResult r;
+  try {
+    c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(device));
+    int64_t visits = 0;
+    check(rt_count_visits(&c, lens.data(), static_cast<int>(lens.size()), &visits));
+    int64_t n_blocks = 0;
+    for (int32_t n : lens) n_blocks += n / 64;
+    std::vector<int32_t> kv_ptr(n_blocks + 1), kv_idx(static_cast<size_t>(visits) * c.heads);
+    check(rt_build_block_csr(&c, seed, lens.data(), static_cast<int>(lens.size()), kv_ptr.data(), kv_idx.data()));
+    auto side = c10::cuda::getStreamFromPool(false, static_cast<c10::DeviceIndex>(device));
+    check(rt_attn_plan_create(&c, lens.data(), static_cast<int>(lens.size()), kv_ptr.data(), kv_idx.data(), 0, -1,
+                              side.stream(), &r.plan));
+  } catch (const std::exception& e) {
+    r.error = e.what();
+  }
+  return r;
+}
+
+// The work list of one batch for all layers with the same block lists: the same model constants, and the same layer
+// index where a sequence is long enough for random blocks.  A program with several models has 12 layers of each
+// registered, whichever of them the batch is for: 6464 tokens with three 12-layer models alive 3764 us a batch with a task per
+// layer, 1784 with one per list (with one model alive 1773).  The partial results of cut lists are part of it: the calls of all layers
+// are ordered on the device (SharedUse).
+class BatchPlan {
+ public:
+  using Key = std::array<int64_t, 9>;
+  static Key key(const rt_config& c, int layer_idx, const std::vector<int32_t>& lens) {
+    bool random = false;
+    for (int32_t n : lens) random |= c.pattern == RT_PATTERN_BIGBIRD && n / 64 > 5 + 2 * c.num_rand;
+    return {c.hidden, c.heads, c.num_rand, c.max_pos, c.pattern, c.band_half, c.dtype, random, random ? layer_idx : 0};
+  }
+  // how: in a task of its own, or (deferred) in the first get()
+  BatchPlan(const rt_config& c, int layer_idx, const std::vector<int32_t>& lens, int device, std::launch how)
+      : device_(device), pending_(std::async(how, build_plan, c, static_cast<uint32_t>(layer_idx), lens, device)) {}
+  ~BatchPlan() { release(nullptr); }
+  BatchPlan(const BatchPlan&) = delete;
+
+  void wait() const {
+    if (pending_.valid()) pending_.wait();
+  }
+  const rt_attn_plan* get() {
+    collect();
+    if (!error_.empty()) throw std::runtime_error(error_);
+    return plan_;
+  }
+  // Gives the memory back: behind `ordered`, a stream that is behind every use (update_meta_data's, under its
+  // SharedUse), or else after a wait for the plan's device.
+  rt_status release(const c10::cuda::CUDAStream* ordered) {
+    collect();
+    rt_attn_plan* plan = std::exchange(plan_, nullptr);
+    if (ordered && ordered->device_index() == device_) return rt_attn_plan_destroy_on(plan, ordered->stream());
+    return rt_attn_plan_destroy(plan);
+  }
+
+ private:
+  void collect() {
+    if (!pending_.valid()) return;
+    PlanResult r = pending_.get();
+    plan_ = r.plan;
+    error_ = std::move(r.error);
+  }
+  int device_;
+  std::future<PlanResult> pending_;
+  rt_attn_plan* plan_ = nullptr;
+  std::string error_;
+};
+
 class BertAttention {
  public:
   BertAttention(torch::Tensor qkv_weight, torch::Tensor qkv_bias, torch::Tensor dense_weight, torch::Tensor dense_bias,
@@ -340,37 +412,23 @@ class BertAttention {
     return c;
   }
 
-  // Host task of one batch: block table of this layer (seeded by its index) -> work list -> upload.
-  PlanResult build_plan(std::vector<int32_t> lens, int device) const {
-    PlanResult r;
-    try {
-      c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(device));
-      const rt_config c = config();
-      int64_t visits = 0;
-      check(rt_count_visits(&c, lens.data(), static_cast<int>(lens.size()), &visits));
-      int64_t n_blocks = 0;
-      for (int32_t n : lens) n_blocks += n / 64;
-      std::vector<int32_t> kv_ptr(n_blocks + 1), kv_idx(static_cast<size_t>(visits) * heads_);
-      check(rt_build_block_csr(&c, static_cast<uint32_t>(layer_idx_), lens.data(), static_cast<int>(lens.size()),
-                               kv_ptr.data(), kv_idx.data()));
-      auto side = c10::cuda::getStreamFromPool(false, static_cast<c10::DeviceIndex>(device));
-      check(rt_attn_plan_create(&c, lens.data(), static_cast<int>(lens.size()), kv_ptr.data(), kv_idx.data(), 0, -1,
-                                side.stream(), &r.plan));
-    } catch (const std::exception& e) {
-      r.error = e.what();
-    }
-    return r;
-  }
-
-  void kick(const std::vector<int32_t>& lens, int device, const c10::cuda::CUDAStream& ordered) {
+  // A new batch; `plans` holds those of the layers before this one.
+  void kick(const std::vector<int32_t>& lens, int device, const c10::cuda::CUDAStream& ordered,
+            std::map<BatchPlan::Key, std::shared_ptr<BatchPlan>>& plans) {
     check(drop_plan(&ordered));
-    if (async_) pending_ = std::async(std::launch::async, &BertAttention::build_plan, this, lens, device);
-    else sync_lens_ = lens;
     device_ = device;
+    if (!async_) {
+      sync_lens_ = lens;
+      return;
+    }
+    const rt_config c = config();
+    auto& shared = plans[BatchPlan::key(c, layer_idx_, lens)];
+    if (!shared) shared = std::make_shared<BatchPlan>(c, layer_idx_, lens, device, std::launch::async);
+    plan_ = shared;
   }
 
   void join() {
-    if (pending_.valid()) pending_.wait();
+    if (plan_) plan_->wait();
   }
 
   // attention_mask and the two partition tensors are not read (the batch is padding-free and the kernel
@@ -407,22 +465,17 @@ class BertAttention {
     }
     // the layer's table: wait for the host task started by MetaData.update_meta_data
     const auto t0 = std::chrono::steady_clock::now();
-    if (pending_.valid()) {
-      PlanResult r = pending_.get();
-      if (!r.error.empty()) throw std::runtime_error(r.error);
-      plan_ = r.plan;
-    } else if (!sync_lens_.empty()) {
-      PlanResult r = build_plan(sync_lens_, device_);
+    if (!plan_ && !sync_lens_.empty()) {
+      plan_ = std::make_shared<BatchPlan>(config(), layer_idx_, sync_lens_, device_, std::launch::deferred);
       sync_lens_.clear();
-      if (!r.error.empty()) throw std::runtime_error(r.error);
-      plan_ = r.plan;
     }
     if (!plan_) throw std::runtime_error("raptor_t: BertAttention called before MetaData.update_meta_data");
+    const rt_attn_plan* plan = plan_->get();
     auto pre = info.find("pre_process");
     if (pre != info.end())
       pre->second += std::chrono::duration<float>(std::chrono::steady_clock::now() - t0).count();
     timed(info, "attention", [&] {
-      check(rt_sparse_attention(ctx.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), plan_, 1.0f, dtype_, st));
+      check(rt_sparse_attention(ctx.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), plan, 1.0f, dtype_, st));
     });
     check(rt_gemm(dense.data_ptr(), ctx.data_ptr(), dense_w_.data_ptr(), nullptr, T, hidden_, hidden_, RT_EPI_NONE,
                   dtype_, st));
@@ -434,24 +487,17 @@ class BertAttention {
   }
 
  private:
-  // Gives the plan back: behind `ordered`, a stream that is behind every use (update_meta_data's, under its
-  // SharedUse), or else after a wait for the plan's device.
+  // The last layer to let go of a plan gives its memory back.
   rt_status drop_plan(const c10::cuda::CUDAStream* ordered) {
-    rt_attn_plan* plan = std::exchange(plan_, nullptr);
-    if (pending_.valid()) {
-      PlanResult r = pending_.get();
-      if (r.plan) rt_attn_plan_destroy(r.plan);
-    }
-    if (ordered && ordered->device_index() == device_) return rt_attn_plan_destroy_on(plan, ordered->stream());
-    return rt_attn_plan_destroy(plan);
+    const std::shared_ptr<BatchPlan> plan = std::exchange(plan_, nullptr);
+    return plan && plan.use_count() == 1 ? plan->release(ordered) : RT_OK;
   }
 
   int heads_, hidden_ = 0, layer_idx_, dtype_ = RT_F16, device_ = 0;
   bool async_;
   torch::Tensor qkv_w_, qkv_b_, dense_w_, dense_b_, ln_w_, ln_b_;
-  std::future<PlanResult> pending_;
   std::vector<int32_t> sync_lens_;
-  rt_attn_plan* plan_ = nullptr;
+  std::shared_ptr<BatchPlan> plan_;
 };
 
 class MetaData {
@@ -489,8 +535,9 @@ class MetaData {
     LayerRegistry::upload(reg.block_seq, bs);
     LayerRegistry::upload(reg.seq_prefix, seq_len_info);
     reg.n_seq = static_cast<int>(lens.size());
+    std::map<BatchPlan::Key, std::shared_ptr<BatchPlan>> plans;
     for (BertAttention* l : reg.layers)
-      if (l) l->kick(lens, device, use.stream());
+      if (l) l->kick(lens, device, use.stream(), plans);
   }
   // layers/metadata.cpp:20-27: shutdown; here: join every pending host task
   void terminate_thread() {
