@@ -417,7 +417,8 @@ rt_status ensure_scratch(rt_encoder* e, int tokens) {
 // FFN down + LayerNorm for batches of few tokens: split-K GEMM into fp32 parts and a LayerNorm that sums them.
 // The cluster kernel walks all K blocks of a row block in sequence, however few row blocks there are (K = 3072:
 // 17.1 us for 128 rows, 17.4 for 1024, 17.9 for 2048, 19.1 for 4096); cut along K until the chip is full, projection
-// and LayerNorm take 9.2 us for 128 rows, 12.3 for 1024, 17.6 for 2048.  Estimates in microseconds, as in plan_gemm
+// and LayerNorm take 10.9 for 512 rows, 12.3 for 1024, 17.6 for 2048; up to 256 rows the split is one over a cluster
+// (plan_gemm), whose sums are one part (256 rows 10.1 -> 8.9 us, 1024 wide 11.1 -> 10.1).  Estimates in microseconds, as in plan_gemm
 // (both sides a little high: the line between them lies at 2048 rows).  With K = 768 or 1024 the parts' traffic eats
 // the gain (8.0 against 6.9 us for 128 rows): not used.
 bool plan_parts(const rt_encoder* e, int K, GemmPlan& plan) {
@@ -427,6 +428,7 @@ bool plan_parts(const rt_encoder* e, int K, GemmPlan& plan) {
   const int max_splits = static_cast<int>(std::min<size_t>(kLnPartsBytes / part, kMaxLnSplits));
   if (max_splits < 1) return false;
   plan = plan_gemm(M, N, K, max_splits, true);
+  if (plan.cluster) return true;  // one part
   const double rows = static_cast<double>(M) * N;
   const double parts_cost = plan.cost + 2.5 + rows * 6 / 6e6;
   double other;
@@ -468,11 +470,18 @@ bool aligned(size_t bytes, std::initializer_list<const void*> ptrs) {
 }
 bool always_fused(const rt_encoder* e, int K) { return e->fuse_layernorm == 2 || (e->cfg.hidden == 768 && K >= 2048); }
 
+// The encoder's weights are written by rt_encoder_set_layer alone, never by a kernel that a forward's may overlap.
+gemm_detail::QkvEpilogue weights_settled() {
+  gemm_detail::QkvEpilogue extra{};
+  extra.settled_w = true;
+  return extra;
+}
+
 rt_status run_parts(rt_encoder* e, const GemmPlan& plan, const char* span, void* out, const void* a, const void* w,
                     const void* bias, const void* residual, const void* gamma, const void* beta, int K, cudaStream_t st) {
   const rt_config& c = e->cfg;
   float* parts = static_cast<float*>(e->ln_parts.p);
-  gemm_detail::QkvEpilogue extra{};
+  gemm_detail::QkvEpilogue extra = weights_settled();
   extra.splits = plan.splits;
   {
     Span s(e, st, span);
@@ -498,7 +507,7 @@ rt_status run_attention(rt_encoder* e, int l, const void* input, void* output, c
   if (e->fuse_qkv) {
     Span s(e, st, "gemm.qkv");
     const int32_t* block_seq = static_cast<const int32_t*>(e->cur->prefix_dev.p) + e->cur->block_seq_off;
-    RT_TRY(rt_gemm_qkv(q, k, v, input, w.qkv_w.p, w.qkv_b.p, block_seq, T, c.heads, H, 0.125f, dt, st));
+    RT_TRY(gemm_qkv_checked(q, k, v, input, w.qkv_w.p, w.qkv_b.p, block_seq, T, c.heads, H, 0.125f, dt, st, true));
   } else {
     {
       Span s(e, st, "gemm.qkv");
@@ -533,7 +542,7 @@ rt_status run_attention(rt_encoder* e, int l, const void* input, void* output, c
   } else {
     {
       Span s(e, st, "gemm.attention_output");
-      RT_TRY(rt_gemm(dense, ctx, w.ao_w.p, nullptr, T, H, H, RT_EPI_NONE, dt, st));
+      RT_TRY(gemm_checked(dense, ctx, w.ao_w.p, nullptr, T, H, H, RT_EPI_NONE, dt, st, weights_settled()));
     }
     Span s(e, st, "add_bias_and_layernorm_kernel");
     RT_TRY(rt_bias_residual_layernorm(output, dense, w.ao_b.p, input, w.aln_g.p, w.aln_b.p, T, H, c.eps, dt, st));
@@ -547,7 +556,8 @@ rt_status run_intermediate(rt_encoder* e, int l, const void* input, void* output
   RT_REQUIRE(w.set, RT_ERR_STATE, "layer %d has no weights", l);
   if (e->fuse_gelu) {
     Span s(e, st, "gemm.ffn_up");
-    RT_TRY(rt_gemm(output, input, w.up_w.p, w.up_b.p, e->tokens, c.ffn, c.hidden, RT_EPI_BIAS_GELU, c.dtype, st));
+    RT_TRY(gemm_checked(output, input, w.up_w.p, w.up_b.p, e->tokens, c.ffn, c.hidden, RT_EPI_BIAS_GELU, c.dtype, st,
+                        weights_settled()));
   } else {
     {
       Span s(e, st, "gemm.ffn_up");

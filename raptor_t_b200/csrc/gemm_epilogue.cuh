@@ -74,26 +74,27 @@ struct QkvEpilogue {
   int heads;
   float q_scale;
   int splits;  // kEpiPartial: parts of K
+  bool settled_w;  // nothing in flight writes W: a kernel may read it before the kernels before it have ended
 };
 constexpr int kEpiQkv = 3;
 // Split-K form: C is fp32 [splits][M][N], part s holds the sum over its K range; no bias.  The reader of the
 // parts (layernorm_parts_kernel) adds them up.
 constexpr int kEpiPartial = 5;
 
-// 32 columns, from `col` on, of one accumulator row: r[] holds the fp32 accumulators, o[] gets the 16-bit results.
-template <bool BF16, int EPI>
+// COLS columns, from `col` on, of one accumulator row: r[] holds the fp32 accumulators, o[] gets the 16-bit results.
+template <bool BF16, int EPI, int COLS = 32>
 __device__ __forceinline__ void epilogue_values(const uint32_t* r, uint32_t* o, int col, int row, int M, int N,
                                                 const uint16_t* __restrict__ bias, const QkvEpilogue& qkv) {
   if constexpr (EPI == RT_EPI_NONE) {
 #pragma unroll
-    for (int j = 0; j < 16; ++j) o[j] = pack2<BF16>(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
+    for (int j = 0; j < COLS / 2; ++j) o[j] = pack2<BF16>(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
   } else {
-    uint32_t res[16];
+    uint32_t res[COLS / 2];
     if constexpr (EPI == RT_EPI_BIAS_RESIDUAL) {
       if (row < M) {
         const uint4* rp = reinterpret_cast<const uint4*>(qkv.residual + static_cast<size_t>(row) * N + col);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
+        for (int q = 0; q < COLS / 8; ++q) {
           const uint4 t = rp[q];
           res[4 * q] = t.x;
           res[4 * q + 1] = t.y;
@@ -102,12 +103,12 @@ __device__ __forceinline__ void epilogue_values(const uint32_t* r, uint32_t* o, 
         }
       } else {
 #pragma unroll
-        for (int q = 0; q < 16; ++q) res[q] = 0u;
+        for (int q = 0; q < COLS / 2; ++q) res[q] = 0u;
       }
     }
     const uint4* bv = reinterpret_cast<const uint4*>(bias + col);
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
+    for (int q = 0; q < COLS / 8; ++q) {
       const uint4 b4 = __ldg(bv + q);
       const uint32_t bw[4] = {b4.x, b4.y, b4.z, b4.w};
 #pragma unroll
@@ -133,36 +134,39 @@ __device__ __forceinline__ void epilogue_values(const uint32_t* r, uint32_t* o, 
   }
 }
 
-// The same, stored by the thread itself.
-template <bool BF16, int EPI>
-__device__ __forceinline__ void epilogue_chunk(const uint32_t* r, int c, int row, int n0, int M, int N,
+// The same, stored by the thread itself.  COLS = 8, 16 or 32: a group never straddles a head.
+template <bool BF16, int EPI, int COLS = 32>
+__device__ __forceinline__ void epilogue_chunk(const uint32_t* r, int col, int row, int M, int N,
                                                uint16_t* __restrict__ C, const uint16_t* __restrict__ bias,
                                                const QkvEpilogue& qkv) {
   if constexpr (EPI == kEpiPartial) {
     if (row < M) {
-      float* dst = reinterpret_cast<float*>(C) + static_cast<size_t>(row) * N + n0 + c * 32;
+      float* dst = reinterpret_cast<float*>(C) + static_cast<size_t>(row) * N + col;
 #pragma unroll
-      for (int q = 0; q < 4; ++q) st_global_v8(dst + 8 * q, r + 8 * q);
+      for (int q = 0; q < COLS / 8; ++q) st_global_v8(dst + 8 * q, r + 8 * q);
     }
     return;
   }
-  uint32_t o[16];
-  epilogue_values<BF16, EPI>(r, o, n0 + c * 32, row, M, N, bias, qkv);
+  uint32_t o[COLS / 2];
+  epilogue_values<BF16, EPI, COLS>(r, o, col, row, M, N, bias, qkv);
   if (row < M) {
     uint16_t* dst;
     if constexpr (EPI == kEpiQkv) {
       const int hidden = qkv.heads * 64;
-      const int n = n0 + c * 32;
-      const int part = n / hidden;
-      const int hcol = n - part * hidden;
+      const int part = col / hidden;
+      const int hcol = col - part * hidden;
       const int2 bs = __ldg(qkv.block_seq + (row >> 6));
       const size_t drow = static_cast<size_t>(bs.x) * qkv.heads + static_cast<size_t>(hcol >> 6) * bs.y + (row - bs.x);
       dst = (part == 0 ? qkv.q : part == 1 ? qkv.k : qkv.v) + drow * 64 + (hcol & 63);
     } else {
-      dst = C + static_cast<size_t>(row) * N + n0 + c * 32;
+      dst = C + static_cast<size_t>(row) * N + col;
     }
-    st_global_v8(dst, o);
-    st_global_v8(dst + 16, o + 8);
+    if constexpr (COLS == 8) {
+      *reinterpret_cast<uint4*>(dst) = make_uint4(o[0], o[1], o[2], o[3]);
+    } else {
+#pragma unroll
+      for (int q = 0; q < COLS / 16; ++q) st_global_v8(dst + 16 * q, o + 8 * q);
+    }
   }
 }
 
@@ -181,8 +185,8 @@ __device__ __forceinline__ void epilogue_row(int width, uint32_t taddr, int row,
     tmem_ld32(taddr + c * 32, r0);
     if (two) tmem_ld32(taddr + (c + 2) * 32, r1);
     tc_wait_ld();
-    epilogue_chunk<BF16, EPI>(r0, c, row, n0, M, N, C, bias, qkv);
-    if (two) epilogue_chunk<BF16, EPI>(r1, c + 2, row, n0, M, N, C, bias, qkv);
+    epilogue_chunk<BF16, EPI>(r0, n0 + c * 32, row, M, N, C, bias, qkv);
+    if (two) epilogue_chunk<BF16, EPI>(r1, n0 + (c + 2) * 32, row, M, N, C, bias, qkv);
   }
 }
 

@@ -13,11 +13,19 @@ struct GemmPlan {
   int width = 64;      // columns of a tile
   int splits = 1;      // parts of K (kEpiPartial only)
   double cost = 0;     // estimated microseconds
+  int cluster = 0;     // > 1: K split over this many CTAs of a cluster (gemm_cluster_sm100.cu)
 };
 
 // Cheapest tiling by the measured costs of the tile shapes; parts: kEpiPartial with up to max_splits parts.
 GemmPlan plan_gemm(int M, int N, int K, int max_splits, bool parts);
 rt_status run_gemm(void* c, const void* a, const void* w, const void* bias, int M, int N, int K, int epi, int dtype,
                    cudaStream_t st, const gemm_detail::QkvEpilogue& extra, const GemmPlan& plan);
+
+// rt_gemm and rt_gemm_qkv; settled_w as in QkvEpilogue.
+rt_status gemm_checked(void* c, const void* a, const void* w, const void* bias, int M, int N, int K, int epilogue,
+                       int dtype, void* stream, const gemm_detail::QkvEpilogue& extra);
+rt_status gemm_qkv_checked(void* q, void* k, void* v, const void* a, const void* w, const void* bias,
+                           const int32_t* block_seq_dev, int M, int heads, int K, float q_scale, int dtype, void* stream,
+                           bool settled_w);
 
 }  // namespace rt

@@ -64,6 +64,7 @@ constexpr TileCost kSingleTiles[3] = {{64, 2.3, 0.2, 0.45}, {128, 2.6, 0.235, 0.
 constexpr TileCost kPairTiles[3] = {{128, 3.6, 0.2, 0.5}, {192, 3.6, 0.24, 1.0}, {256, 3.8, 0.29, 1.2}};
 // the last, partial wave of 256-column pair tiles cut into narrower ones
 constexpr TileCost kTailTiles[2] = {{64, 0, 0.15, 0.5}, {128, 0, 0.2, 0.6}};
+constexpr int kClusterWidth = 64;  // columns of a tile of gemm_cluster_sm100.cu
 constexpr double kPartBytesPerUs = 6e6;  // fp32 parts, written and read through L2
 
 template <int BN>
@@ -263,6 +264,8 @@ rt_status launch_epi(void* c, const void* a, const void* w, const void* bias, in
 
 rt_status gemm_pair_dispatch(void* c, const void* a, const void* w, const void* bias, int M, int N, int K, int epi,
                              bool bf16, cudaStream_t st, const gemm_detail::QkvEpilogue& qkv, int main_tiles, int tail_w);
+rt_status gemm_cluster_dispatch(void* c, const void* a, const void* w, const void* bias, int M, int N, int K, int epi,
+                                bool bf16, cudaStream_t st, const gemm_detail::QkvEpilogue& extra, int cluster);
 
 GemmPlan plan_gemm(int M, int N, int K, int max_splits, bool to_parts) {
   const int sms = gemm_sm_count(), pairs = sms / 2;
@@ -287,12 +290,23 @@ GemmPlan plan_gemm(int M, int N, int K, int max_splits, bool to_parts) {
     for (const TileCost& c : kTailTiles)
       consider(kPairTiles[2].at(full, kbs) + c.at(waves(rest * (256 / c.width), pairs), kbs), true, full * pairs, c.width);
   }
+  // Two rows of tiles at most and K long enough to be worth sharing: split over clusters, as far as that leaves SMs for
+  // the kernel behind to be resident early (in the chain of a forward, 12 layers: 128 rows 446 -> 381 us, 256 rows
+  // 481 -> 441; with 4 CTAs for each of 36 or 48 tiles 428, for each of the 36 tiles of 384 rows 495 -> 531).  Alone, weights
+  // from HBM, us: 128 rows 768 x 768 5.9 -> 4.8, 3072 x 768 6.3 -> 5.6, 768 x 3072 13.1 -> 5.9, 1024 x 4096 16.4 -> 7.7;
+  // 256 rows 2304 x 768 6.0 -> 5.3, 768 x 3072 13.0 -> 6.8.
+  if (M <= 2 * kBM && K >= 8 * kBK) {
+    const int tiles = mt * (N / kClusterWidth);
+    const int cluster = tiles * 8 <= 96 ? 8 : tiles * 4 <= 128 ? 4 : tiles * 2 <= sms ? 2 : 0;
+    if (cluster) best = GemmPlan{false, 0, kClusterWidth, 1, 3.0, cluster};
+  }
   return best;
 }
 
 rt_status run_gemm(void* c, const void* a, const void* w, const void* bias, int M, int N, int K, int epi, int dtype,
                    cudaStream_t st, const gemm_detail::QkvEpilogue& extra, const GemmPlan& plan) {
   const bool bf = dtype == RT_BF16;
+  if (plan.cluster) return gemm_cluster_dispatch(c, a, w, bias, M, N, K, epi, bf, st, extra, plan.cluster);
   if (plan.pair) return gemm_pair_dispatch(c, a, w, bias, M, N, K, epi, bf, st, extra, plan.main_tiles, plan.width);
   if (plan.width == 256) return bf ? launch_epi<256, true>(c, a, w, bias, M, N, K, epi, st, extra)
                                    : launch_epi<256, false>(c, a, w, bias, M, N, K, epi, st, extra);
@@ -302,12 +316,8 @@ rt_status run_gemm(void* c, const void* a, const void* w, const void* bias, int 
             : launch_epi<64, false>(c, a, w, bias, M, N, K, epi, st, extra);
 }
 
-}  // namespace rt
-
-using namespace rt;
-
-static rt_status gemm_entry(void* c, const void* a, const void* w, const void* bias, int M, int N, int K, int epilogue,
-                            int dtype, void* stream, const gemm_detail::QkvEpilogue& extra) {
+rt_status gemm_checked(void* c, const void* a, const void* w, const void* bias, int M, int N, int K, int epilogue,
+                       int dtype, void* stream, const gemm_detail::QkvEpilogue& extra) {
   RT_REQUIRE(c && a && w, RT_ERR_INVALID, "gemm: null pointer");
   RT_REQUIRE(M >= 0 && N > 0 && K > 0 && N % 64 == 0 && K % 64 == 0, RT_ERR_INVALID,
              "gemm: need N %% 64 == 0 and K %% 64 == 0 (got M=%d N=%d K=%d)", M, N, K);
@@ -320,25 +330,9 @@ static rt_status gemm_entry(void* c, const void* a, const void* w, const void* b
   return run_gemm(c, a, w, bias, M, N, K, epilogue, dtype, static_cast<cudaStream_t>(stream), extra, plan_gemm(M, N, K, 1, false));
 }
 
-extern "C" rt_status rt_gemm(void* c, const void* a, const void* w, const void* bias, int M, int N, int K, int epilogue,
-                             int dtype, void* stream) {
-  RT_REQUIRE(epilogue == RT_EPI_NONE || epilogue == RT_EPI_BIAS || epilogue == RT_EPI_BIAS_GELU, RT_ERR_INVALID,
-             "gemm: unknown epilogue %d", epilogue);
-  return gemm_entry(c, a, w, bias, M, N, K, epilogue, dtype, stream, gemm_detail::QkvEpilogue{});
-}
-
-extern "C" rt_status rt_gemm_residual(void* c, const void* a, const void* w, const void* bias, const void* residual,
-                                      int M, int N, int K, int dtype, void* stream) {
-  RT_REQUIRE(residual != nullptr && (reinterpret_cast<uintptr_t>(residual) & 15u) == 0, RT_ERR_INVALID,
-             "gemm_residual: residual must be a 16-byte aligned device pointer");
-  gemm_detail::QkvEpilogue e{};
-  e.residual = static_cast<const uint16_t*>(residual);
-  return gemm_entry(c, a, w, bias, M, N, K, RT_EPI_BIAS_RESIDUAL, dtype, stream, e);
-}
-
-extern "C" rt_status rt_gemm_qkv(void* q, void* k, void* v, const void* a, const void* w, const void* bias,
-                                 const int32_t* block_seq_dev, int M, int heads, int K, float q_scale, int dtype,
-                                 void* stream) {
+rt_status gemm_qkv_checked(void* q, void* k, void* v, const void* a, const void* w, const void* bias,
+                           const int32_t* block_seq_dev, int M, int heads, int K, float q_scale, int dtype, void* stream,
+                           bool settled_w) {
   RT_REQUIRE(q && k && v && a && w && bias && block_seq_dev, RT_ERR_INVALID, "gemm_qkv: null pointer");
   const int N = 3 * heads * 64;
   RT_REQUIRE(M >= 0 && M % 64 == 0 && heads > 0 && K > 0 && K % 64 == 0, RT_ERR_INVALID,
@@ -351,7 +345,33 @@ extern "C" rt_status rt_gemm_qkv(void* q, void* k, void* v, const void* a, const
   if (M == 0) return RT_OK;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   QkvEpilogue e{nullptr, (uint16_t*)q, (uint16_t*)k, (uint16_t*)v, reinterpret_cast<const int2*>(block_seq_dev), heads,
-                q_scale, 1};
+                q_scale, 1, settled_w};
   // every tile width keeps a 32-column chunk inside one head
   return run_gemm(nullptr, a, w, bias, M, N, K, kEpiQkv, dtype, st, e, plan_gemm(M, N, K, 1, false));
+}
+
+}  // namespace rt
+
+using namespace rt;
+
+extern "C" rt_status rt_gemm(void* c, const void* a, const void* w, const void* bias, int M, int N, int K, int epilogue,
+                             int dtype, void* stream) {
+  RT_REQUIRE(epilogue == RT_EPI_NONE || epilogue == RT_EPI_BIAS || epilogue == RT_EPI_BIAS_GELU, RT_ERR_INVALID,
+             "gemm: unknown epilogue %d", epilogue);
+  return gemm_checked(c, a, w, bias, M, N, K, epilogue, dtype, stream, gemm_detail::QkvEpilogue{});
+}
+
+extern "C" rt_status rt_gemm_residual(void* c, const void* a, const void* w, const void* bias, const void* residual,
+                                      int M, int N, int K, int dtype, void* stream) {
+  RT_REQUIRE(residual != nullptr && (reinterpret_cast<uintptr_t>(residual) & 15u) == 0, RT_ERR_INVALID,
+             "gemm_residual: residual must be a 16-byte aligned device pointer");
+  gemm_detail::QkvEpilogue e{};
+  e.residual = static_cast<const uint16_t*>(residual);
+  return gemm_checked(c, a, w, bias, M, N, K, RT_EPI_BIAS_RESIDUAL, dtype, stream, e);
+}
+
+extern "C" rt_status rt_gemm_qkv(void* q, void* k, void* v, const void* a, const void* w, const void* bias,
+                                 const int32_t* block_seq_dev, int M, int heads, int K, float q_scale, int dtype,
+                                 void* stream) {
+  return gemm_qkv_checked(q, k, v, a, w, bias, block_seq_dev, M, heads, K, q_scale, dtype, stream, false);
 }
