@@ -175,7 +175,8 @@ struct rt_encoder {
     bool forward_recorded = false;
     bool uploads_recorded = false;
     bool used = false;
-    std::vector<cudaEvent_t> table_ready;
+    std::vector<cudaEvent_t> table_ready;  // that of the last layer of an upload stands for all of them
+    std::vector<int> upload_end;           // per layer: the last layer of its upload
   } slots[kSlots];
   uint64_t batch_counter = 0;
   Slot* cur = nullptr;
@@ -272,9 +273,13 @@ struct Span {
 };
 
 // One batch: per layer, per-sequence templates (cached across batches) -> work list -> pinned
-// region -> one asynchronous upload -> event.
+// region -> asynchronous upload -> event.  Lists so short that building all of them takes no longer than a few uploads go
+// over in one copy: copies, events and waits of twelve layers are a quarter of the host's work for a single short sequence.
+constexpr size_t kOneUploadBytes = 64u << 10;
 void build_batch_metadata(rt_encoder* e) {
   rt_encoder::Slot& slot = *e->cur;
+  const bool one_upload = e->region_bytes * e->cfg.layers <= kOneUploadBytes;
+  int upload_begin = 0;  // first layer that is not on its way
   std::vector<const SeqTemplate*> tmpl(e->n_seq);
   AttnPlanHost refill;
   for (int l = 0; l < e->cfg.layers; ++l) {
@@ -305,9 +310,9 @@ void build_batch_metadata(rt_encoder* e) {
         plan = &refill;
       }
     }
+    const bool upload = !one_upload || l + 1 == e->cfg.layers;
     if (s == RT_OK) {
       uint8_t* host = slot.meta_pinned + static_cast<size_t>(l) * e->region_bytes;
-      uint8_t* dev = static_cast<uint8_t*>(slot.meta_dev.p) + static_cast<size_t>(l) * e->region_bytes;
       const size_t items_b = plan->items.size() * sizeof(AttnItem);
       const size_t entries_b = plan->entries.size() * sizeof(int32_t);
       const size_t cta_b = plan->cta_ptr.size() * sizeof(int32_t);
@@ -323,9 +328,16 @@ void build_batch_metadata(rt_encoder* e) {
         std::memcpy(host + e->cta_off, plan->cta_ptr.data(), cta_b);
         std::memcpy(host + e->groups_off, plan->groups.data(), groups_b);
         e->plan_groups[l] = static_cast<int>(plan->groups.size() / 6);
-        // one copy for the whole region of the layer (items | entries | per-CTA offsets | groups)
-        cudaError_t ce = cudaMemcpyAsync(dev, host, e->groups_off + groups_b, cudaMemcpyHostToDevice, e->meta_stream);
-        if (ce == cudaSuccess) ce = cudaEventRecord(slot.table_ready[l], e->meta_stream);
+        // one copy for the whole region of a layer (items | entries | per-CTA offsets | groups), or of several
+        cudaError_t ce = cudaSuccess;
+        if (upload) {
+          const size_t first = upload_begin * e->region_bytes;
+          ce = cudaMemcpyAsync(static_cast<uint8_t*>(slot.meta_dev.p) + first, slot.meta_pinned + first,
+                               (l - upload_begin) * e->region_bytes + e->groups_off + groups_b, cudaMemcpyHostToDevice,
+                               e->meta_stream);
+          if (ce == cudaSuccess) ce = cudaEventRecord(slot.table_ready[l], e->meta_stream);
+          for (; upload_begin <= l; ++upload_begin) slot.upload_end[upload_begin] = l;
+        }
         if (ce == cudaSuccess && l + 1 == e->cfg.layers) {
           ce = cudaEventRecord(slot.uploads_done, e->meta_stream);
           slot.uploads_recorded = ce == cudaSuccess;
@@ -348,10 +360,10 @@ void build_batch_metadata(rt_encoder* e) {
         e->worker_error = last_error_ref();
         e->layers_recorded = e->cfg.layers;  // release every waiter; they will see the status
       } else {
-        e->layers_recorded = l + 1;
+        e->layers_recorded = upload_begin;
       }
     }
-    e->cv.notify_all();
+    if (s != RT_OK || upload) e->cv.notify_all();
     if (s != RT_OK) return;
   }
 }
@@ -372,15 +384,27 @@ void worker_main(rt_encoder* e) {
   }
 }
 
-rt_status wait_layer_table(rt_encoder* e, int layer, cudaStream_t st) {
+// What a forward's stream has waited for.  Uploads stand in layer order on one stream, so the wait for one covers every
+// earlier one.
+struct UploadsSeen {
+  int tables = 0;  // of layers [0, tables)
+};
+
+// The first layer of a forward waits for its own table, which is the first to arrive; a later one for the last that is
+// on its way: a forward then has two or three waits instead of two per layer.
+rt_status wait_layer_table(rt_encoder* e, int layer, cudaStream_t st, UploadsSeen* seen) {
+  if (seen && seen->tables > layer) return RT_OK;
   auto t0 = std::chrono::steady_clock::now();
+  int last = layer;
   {
     std::unique_lock<std::mutex> lk(e->mu);
     e->cv.wait(lk, [&] { return e->layers_recorded > layer; });
     if (e->worker_status != RT_OK) return fail(e->worker_status, "metadata worker: %s", e->worker_error.c_str());
+    last = seen && seen->tables > 0 ? e->layers_recorded - 1 : e->cur->upload_end[layer];
   }
   e->pre_process_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
-  RT_CHECK_CUDA(cudaStreamWaitEvent(st, e->cur->table_ready[layer], 0));
+  RT_CHECK_CUDA(cudaStreamWaitEvent(st, e->cur->table_ready[last], 0));
+  if (seen) seen->tables = last + 1;
   return RT_OK;
 }
 
@@ -491,8 +515,10 @@ rt_status run_parts(rt_encoder* e, const GemmPlan& plan, const char* span, void*
   return layernorm_parts(out, parts, plan.splits, bias, residual, gamma, beta, e->tokens, c.hidden, c.eps, c.dtype, st);
 }
 
-// attention sub-layer: out = LN(ctx W_o + b_o + input)
-rt_status run_attention(rt_encoder* e, int l, const void* input, void* output, cudaStream_t st) {
+// attention sub-layer: out = LN(ctx W_o + b_o + input).  seen: inside a forward, whose stream has waited for the prefix
+// upload; a call of its own (nullptr) waits for what it needs.
+rt_status run_attention(rt_encoder* e, int l, const void* input, void* output, cudaStream_t st,
+                        UploadsSeen* seen = nullptr) {
   const rt_config& c = e->cfg;
   LayerWeights& w = e->layers[l];
   RT_REQUIRE(w.set, RT_ERR_STATE, "layer %d has no weights", l);
@@ -503,7 +529,7 @@ rt_status run_attention(rt_encoder* e, int l, const void* input, void* output, c
   void* v = e->scratch["v_out"].p;
   void* ctx = e->scratch["attention_out"].p;
   void* dense = e->scratch["dense_out"].p;
-  RT_CHECK_CUDA(cudaStreamWaitEvent(st, e->cur->prefix_ready, 0));
+  if (!seen) RT_CHECK_CUDA(cudaStreamWaitEvent(st, e->cur->prefix_ready, 0));
   if (e->fuse_qkv) {
     Span s(e, st, "gemm.qkv");
     const int32_t* block_seq = static_cast<const int32_t*>(e->cur->prefix_dev.p) + e->cur->block_seq_off;
@@ -517,7 +543,7 @@ rt_status run_attention(rt_encoder* e, int l, const void* input, void* output, c
     RT_TRY(rt_qkv_bias_transpose(qkv, w.qkv_b.p, q, k, v, (const int32_t*)e->cur->prefix_dev.p, e->n_seq, e->n_blocks,
                                  c.heads, 0.125f, dt, st));
   }
-  RT_TRY(wait_layer_table(e, l, st));
+  RT_TRY(wait_layer_table(e, l, st, seen));
   {
     Span s(e, st, "attention");
     const uint8_t* dev = static_cast<const uint8_t*>(e->cur->meta_dev.p) + static_cast<size_t>(l) * e->region_bytes;
@@ -661,6 +687,7 @@ extern "C" rt_status rt_encoder_create(const rt_config* cfg, rt_encoder** out) {
     cudaEventCreateWithFlags(&slot.uploads_done, cudaEventDisableTiming);
     slot.table_ready.resize(cfg->layers);
     for (auto& ev : slot.table_ready) cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+    slot.upload_end.assign(cfg->layers, 0);
   }
   e->worker = std::thread(worker_main, e);
   *out = e;
@@ -916,8 +943,9 @@ rt_status end_forward(rt_encoder* e, cudaStream_t st) {
 rt_status run_layers(rt_encoder* e, void* hidden, int l0, int l1, cudaStream_t st) {
   void* attn_out = e->scratch["attention_output"].p;
   void* ffn = e->scratch["intermediate"].p;
+  UploadsSeen seen;
   for (int l = l0; l < l1; ++l) {
-    RT_TRY(run_attention(e, l, hidden, attn_out, st));
+    RT_TRY(run_attention(e, l, hidden, attn_out, st, &seen));
     RT_TRY(run_intermediate(e, l, attn_out, ffn, st));
     RT_TRY(run_output(e, l, ffn, attn_out, hidden, st));
   }
