@@ -279,8 +279,9 @@ sparse_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
   tc_fence_after_sync();
   const uint32_t tmem_base = sm.tmem_slot;
   AbortCtx ab{&sm.abort_flag, error_flag};
-  RT_PDL_WAIT();  // q/k/v, the work list and the output buffer belong to earlier work until here
-
+  // The work list is on the device before this kernel can start (uploads are waited for by the host or by the stream, never
+  // written by the kernel before): its first reads, three dependent ones, overlap the end of that kernel.  q/k/v, the
+  // output and the partial results belong to earlier work until each role's griddepcontrol.wait.
   const int item_begin = cta_ptr[blockIdx.x];
   const int item_end = cta_ptr[blockIdx.x + 1];
 
@@ -313,6 +314,7 @@ sparse_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         uint32_t e_g = 0, step = 0, itn = 0;
         AttnItem it = items[item_begin];
         bool ok = true;
+        RT_PDL_WAIT();
         for (int idx = item_begin; ok && idx < item_end; ++idx) {
           AttnItem nxt{};
           if (idx + 1 < item_end) nxt = items[idx + 1];  // in flight while this item's steps are issued
@@ -459,6 +461,7 @@ sparse_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       return hi;
     };
     int4 next_item = item_begin < item_end ? load_item(item_begin) : make_int4(0, 0, 0, 0);
+    RT_PDL_WAIT();
     for (int it = item_begin; it < item_end && ok; ++it) {
       const int4 item = next_item;
       if (it + 1 < item_end) next_item = load_item(it + 1);  // in flight while this item is processed
@@ -623,12 +626,12 @@ __global__ void __launch_bounds__(8 * kMergeRows) merge_partials_kernel(uint16_t
                                                                         const float* __restrict__ part_o,
                                                                         const float* __restrict__ part_ml, int hidden) {
   RT_PDL_LAUNCH_DEPENDENTS();
-  RT_PDL_WAIT();
   const int32_t* g = groups + blockIdx.x * 6;
   const int first = g[0], parts = g[1], head = g[4] & 255;
   const int row = blockIdx.y * kMergeRows + (threadIdx.x >> 3);
   const int col = (threadIdx.x & 7) * 8;
   const int tok0 = row < 64 ? g[2] : g[3];
+  RT_PDL_WAIT();  // the list is older than the attention kernel, its partial results are not
   if (tok0 < 0) return;
   const float2* ml = reinterpret_cast<const float2*>(part_ml) + static_cast<size_t>(first) * 128 + row;
   const float* src = part_o + (static_cast<size_t>(first) * 128 + row) * 64 + col;
