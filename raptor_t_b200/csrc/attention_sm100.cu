@@ -250,6 +250,9 @@ sparse_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
   }
 
   if (threadIdx.x == 0) {
+    prefetch_tensormap(&map_q);  // their fetch overlaps the end of the kernel before, too
+    prefetch_tensormap(&map_k);
+    prefetch_tensormap(&map_v);
     for (int i = 0; i < 2; ++i) {
       mbar_init(&sm.q_full[i], 1);
       mbar_init(&sm.q_empty[i], 1);
@@ -293,9 +296,6 @@ sparse_attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       // asynchronous copies issued kEntAhead entries early, the next item is prefetched in
       // registers.  A CTA's items are consecutive and so are their lists.
       if (lane == 0 && item_begin < item_end) {
-        prefetch_tensormap(&map_q);
-        prefetch_tensormap(&map_k);
-        prefetch_tensormap(&map_v);
         const int ent_first = items[item_begin].entry_off;
         const AttnItem& zi = items[item_end - 1];
         const uint32_t total = static_cast<uint32_t>(zi.entry_off + zi.n_entries - ent_first);

@@ -75,6 +75,8 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   const int kb0 = rank * k_blocks / S, n_kb = (rank + 1) * k_blocks / S - kb0;
 
   if (threadIdx.x == 0) {
+    prefetch_tensormap(&map_a);  // their fetch overlaps the end of the kernel before, too
+    prefetch_tensormap(&map_w);
     for (int s = 0; s < kStages; ++s) {
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);

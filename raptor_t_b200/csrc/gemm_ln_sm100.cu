@@ -181,6 +181,10 @@ gemm_ln_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   auto peer_of = [&](int t) { return PAIR ? static_cast<uint32_t>(2 * t) + hrow : static_cast<uint32_t>(t); };
 
   if (threadIdx.x == 0) {
+    prefetch_tensormap(&map_a);  // their fetch overlaps the end of the kernel before, too
+    prefetch_tensormap(&map_w);
+    prefetch_tensormap(&map_res);
+    prefetch_tensormap(&map_out);
     for (int s = 0; s < kStages; ++s) {
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
@@ -219,8 +223,6 @@ gemm_ln_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   if (warp == 0) {
     // ------------------------------------------------------------- TMA producer (every CTA)
     if (lane == 0) {
-      prefetch_tensormap(&map_a);
-      prefetch_tensormap(&map_w);
       uint32_t it = 0;
       bool ok = true;
       const int n0 = tile * TW + hrow * Cfg::kWRows;

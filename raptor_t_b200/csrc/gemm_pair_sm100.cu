@@ -66,6 +66,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   const int n_pairs = gridDim.x >> 1;
 
   if (threadIdx.x == 0) {
+    prefetch_tensormap(&map_a);  // their fetch overlaps the end of the kernel before, too
+    prefetch_tensormap(&map_w);
+    prefetch_tensormap(&map_wt);
+    prefetch_tensormap(&map_c);
     for (int s = 0; s < kStages; ++s) {
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
@@ -119,9 +123,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   if (warp == 0) {
     // ------------------------------------------------------------- TMA producer (both CTAs)
     if (lane == 0) {
-      prefetch_tensormap(&map_a);
-      prefetch_tensormap(&map_w);
-      prefetch_tensormap(&map_wt);
       uint32_t it = 0;
       bool ok = true;
       for (int t = pair; t < n_tiles && ok; t += n_pairs) {

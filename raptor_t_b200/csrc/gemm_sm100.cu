@@ -99,6 +99,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
   const int lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
+    prefetch_tensormap(&map_a);  // their fetch overlaps the end of the kernel before, too
+    prefetch_tensormap(&map_w);
     for (int s = 0; s < Cfg::kStages; ++s) {
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
@@ -141,8 +143,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
   if (warp == 0) {
     // ------------------------------------------------------------- TMA producer
     if (lane == 0) {
-      prefetch_tensormap(&map_a);
-      prefetch_tensormap(&map_w);
       uint32_t it = 0;
       bool ok = true;
       for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
