@@ -556,8 +556,7 @@ rt_status run_attention(rt_encoder* e, int l, const void* input, void* output, c
   }
   if (fuses_layernorm(e, H) && (always_fused(e, H) || aligned(32, {output, input}))) {
     Span s(e, st, "gemm.attention_output");
-    RT_TRY(rt_gemm_bias_residual_layernorm(output, ctx, w.ao_w.p, w.ao_b.p, input, w.aln_g.p, w.aln_b.p, T, H, H, c.eps,
-                                           dt, st));
+    RT_TRY(gemm_layernorm_checked(output, ctx, w.ao_w.p, w.ao_b.p, input, w.aln_g.p, w.aln_b.p, T, H, H, c.eps, dt, st, true));
   } else if (e->fuse_residual) {
     {
       Span s(e, st, "gemm.attention_output");
@@ -609,8 +608,8 @@ rt_status run_output(rt_encoder* e, int l, const void* ffn, const void* residual
   }
   if (fuses_layernorm(e, c.ffn) && (always_fused(e, c.ffn) || aligned(32, {ffn, residual, out}))) {
     Span s(e, st, "gemm.ffn_down");
-    return rt_gemm_bias_residual_layernorm(out, ffn, w.down_w.p, w.down_b.p, residual, w.oln_g.p, w.oln_b.p, e->tokens,
-                                           c.hidden, c.ffn, c.eps, c.dtype, st);
+    return gemm_layernorm_checked(out, ffn, w.down_w.p, w.down_b.p, residual, w.oln_g.p, w.oln_b.p, e->tokens, c.hidden, c.ffn,
+                                  c.eps, c.dtype, st, true);
   }
   if (e->fuse_residual) {
     {

@@ -149,7 +149,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 gemm_ln_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                const __grid_constant__ CUtensorMap map_res, const __grid_constant__ CUtensorMap map_out,
                const uint16_t* __restrict__ bias, const uint16_t* __restrict__ gamma, const uint16_t* __restrict__ beta,
-               int M, int K, float eps, int* error_flag) {
+               int M, int K, float eps, bool settled_w, int* error_flag) {
   using Cfg = LnCfg<PAIR, NT, TW>;
   constexpr int N = Cfg::kN, kStages = Cfg::kStages, kStageBytes = Cfg::kStageBytes;
   constexpr int kTileN = 256;  // TMEM columns between the two accumulators
@@ -212,12 +212,27 @@ gemm_ln_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   cluster_arrive();  // every peer's barriers exist before anything remote touches them
   cluster_wait();
   tc_fence_after_sync();
+  const int n_tiles_m = (M + Cfg::kRows - 1) / Cfg::kRows;
+  const int k_blocks = K / kBK;
+  const int w_row0 = tile * TW + hrow * Cfg::kWRows;
+  // W of the first ring fill, where nothing in flight writes it: it comes from HBM while the kernel before still runs
+  // (12 layers, 4096 tokens: with the same in gemm_pair_sm100.cu 1158 -> 1145 us)
+  uint32_t w_ahead = 0;
+  if (settled_w && threadIdx.x == 0) {
+    for (; w_ahead < kStages && static_cast<int>(w_ahead) < k_blocks; ++w_ahead) {
+      uint8_t* sw = smem + w_ahead * kStageBytes + kABytes;
+      if constexpr (PAIR) {
+        if (hrow == 0) mbar_arrive_expect_tx(&full[w_ahead], 2 * kStageBytes);
+        tma_load_2d_to_leader(sw, &map_w, w_ahead * kBK, w_row0, map_to_rank(&full[w_ahead], leader));
+      } else {
+        mbar_arrive_expect_tx(&full[w_ahead], kStageBytes);
+        tma_load_2d(sw, &map_w, w_ahead * kBK, w_row0, &full[w_ahead]);
+      }
+    }
+  }
   RT_PDL_WAIT();  // operands, parameters, residual and the output buffer belong to the previous kernel until here
   const uint32_t tmem_base = *tmem_slot;
   AbortCtx ab{cta_abort, error_flag};
-
-  const int n_tiles_m = (M + Cfg::kRows - 1) / Cfg::kRows;
-  const int k_blocks = K / kBK;
 
   if (warp < 4) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsIssue));
   if (warp == 0) {
@@ -225,7 +240,6 @@ gemm_ln_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     if (lane == 0) {
       uint32_t it = 0;
       bool ok = true;
-      const int n0 = tile * TW + hrow * Cfg::kWRows;
       for (int t = cluster_id; t < n_tiles_m && ok; t += n_clusters) {
         const int m0 = t * Cfg::kRows + hrow * 128;
         for (int kb = 0; kb < k_blocks; ++kb, ++it) {
@@ -234,14 +248,14 @@ gemm_ln_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           if (!mbar_wait(&empty[s], ph ^ 1, ab, 121)) { ok = false; break; }
           uint8_t* sa = smem + s * kStageBytes;
           if constexpr (PAIR) {
-            if (hrow == 0) mbar_arrive_expect_tx(&full[s], 2 * kStageBytes);  // both CTAs' bytes
+            if (hrow == 0 && it >= w_ahead) mbar_arrive_expect_tx(&full[s], 2 * kStageBytes);  // both CTAs' bytes
             const uint32_t leader_bar = map_to_rank(&full[s], leader);
             tma_load_2d_to_leader(sa, &map_a, kb * kBK, m0, leader_bar);
-            tma_load_2d_to_leader(sa + kABytes, &map_w, kb * kBK, n0, leader_bar);
+            if (it >= w_ahead) tma_load_2d_to_leader(sa + kABytes, &map_w, kb * kBK, w_row0, leader_bar);
           } else {
-            mbar_arrive_expect_tx(&full[s], kStageBytes);
+            if (it >= w_ahead) mbar_arrive_expect_tx(&full[s], kStageBytes);
             tma_load_2d(sa, &map_a, kb * kBK, m0, &full[s]);
-            tma_load_2d(sa + kABytes, &map_w, kb * kBK, n0, &full[s]);
+            if (it >= w_ahead) tma_load_2d(sa + kABytes, &map_w, kb * kBK, w_row0, &full[s]);
           }
         }
       }
@@ -498,7 +512,7 @@ int resident_clusters() {
 
 template <bool BF16, bool PAIR, int NT, int TW>
 rt_status launch_ln(void* out, const void* a, const void* w, const void* bias, const void* residual, const void* gamma,
-                    const void* beta, int M, int K, float eps, cudaStream_t st) {
+                    const void* beta, int M, int K, float eps, bool settled_w, cudaStream_t st) {
   using Cfg = LnCfg<PAIR, NT, TW>;
   constexpr int kSmemBytes = Cfg::kSmemBytes;
   static_assert(kSmemBytes <= 227 * 1024, "shared memory of one CTA");
@@ -529,7 +543,7 @@ rt_status launch_ln(void* out, const void* a, const void* w, const void* bias, c
   cfg.numAttrs = 2;
   RT_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, ma, mw, mr, mo, static_cast<const uint16_t*>(bias),
                                    static_cast<const uint16_t*>(gamma), static_cast<const uint16_t*>(beta), M, K, eps,
-                                   err));
+                                   settled_w, err));
   count_launch();
   RT_CHECK_CUDA(cudaGetLastError());
   return RT_OK;
@@ -538,12 +552,10 @@ rt_status launch_ln(void* out, const void* a, const void* w, const void* bias, c
 }  // namespace
 }  // namespace rt
 
-using namespace rt;
-
-extern "C" rt_status rt_gemm_bias_residual_layernorm(void* out_dev, const void* a_dev, const void* w_dev,
-                                                     const void* bias_dev, const void* residual_dev,
-                                                     const void* gamma_dev, const void* beta_dev, int M, int N, int K,
-                                                     float eps, int dtype, void* stream) {
+namespace rt {
+rt_status gemm_layernorm_checked(void* out_dev, const void* a_dev, const void* w_dev, const void* bias_dev,
+                                 const void* residual_dev, const void* gamma_dev, const void* beta_dev, int M, int N, int K,
+                                 float eps, int dtype, void* stream, bool settled_w) {
   RT_REQUIRE(out_dev && a_dev && w_dev && bias_dev && residual_dev && gamma_dev && beta_dev, RT_ERR_INVALID,
              "gemm_layernorm: null pointer");
   RT_REQUIRE(N == 768 || N == 1024, RT_ERR_UNSUPPORTED, "gemm_layernorm: N must be 768 or 1024 (got %d)", N);
@@ -562,12 +574,21 @@ extern "C" rt_status rt_gemm_bias_residual_layernorm(void* out_dev, const void* 
   const bool bf = dtype == RT_BF16;
   const int blocks = (M + 127) / 128;
 #define RT_LN_LAUNCH(PAIR, NT, TW)                                                                                  \
-  (bf ? launch_ln<true, PAIR, NT, TW>(out_dev, a_dev, w_dev, bias_dev, residual_dev, gamma_dev, beta_dev, M, K, eps, st) \
-      : launch_ln<false, PAIR, NT, TW>(out_dev, a_dev, w_dev, bias_dev, residual_dev, gamma_dev, beta_dev, M, K, eps, st))
+  (bf ? launch_ln<true, PAIR, NT, TW>(out_dev, a_dev, w_dev, bias_dev, residual_dev, gamma_dev, beta_dev, M, K, eps, settled_w, st) \
+      : launch_ln<false, PAIR, NT, TW>(out_dev, a_dev, w_dev, bias_dev, residual_dev, gamma_dev, beta_dev, M, K, eps, settled_w, st))
   if (N == 768) {
     if (blocks <= resident_clusters<true, false, 4, 192>()) return RT_LN_LAUNCH(false, 4, 192);
     return RT_LN_LAUNCH(true, 3, 256);
   }
   return RT_LN_LAUNCH(true, 4, 256);
 #undef RT_LN_LAUNCH
+}
+}  // namespace rt
+
+extern "C" rt_status rt_gemm_bias_residual_layernorm(void* out_dev, const void* a_dev, const void* w_dev,
+                                                     const void* bias_dev, const void* residual_dev,
+                                                     const void* gamma_dev, const void* beta_dev, int M, int N, int K,
+                                                     float eps, int dtype, void* stream) {
+  return rt::gemm_layernorm_checked(out_dev, a_dev, w_dev, bias_dev, residual_dev, gamma_dev, beta_dev, M, N, K, eps, dtype,
+                                    stream, false);
 }

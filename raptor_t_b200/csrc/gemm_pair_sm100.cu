@@ -90,10 +90,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   cluster_arrive();  // the peer's barriers exist before anything remote touches them
   cluster_wait();
   tc_fence_after_sync();
-  RT_PDL_WAIT();  // operands and the output buffer belong to the previous kernel until here
-  const uint32_t tmem_base = *tmem_slot;
-  AbortCtx ab{cta_abort, error_flag};
-
   const int n_tiles_m = (M + kTileM - 1) / kTileM;
   const int tail_n = N / tail_w;                      // tiles of tail_w columns per row block
   const int tail0 = main_tiles ? main_tiles * (kTileN / tail_w) : 0;  // of these, covered by the main tiles
@@ -120,6 +116,21 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     return r;
   };
 
+  // W of the first ring fill, where nothing in flight writes it: it comes from HBM while the kernel before still runs
+  uint32_t w_ahead = 0;
+  if (qkv.settled_w && threadIdx.x == 0) {
+    const Tile tl = tile_of(pair);
+    const CUtensorMap* mw = pair % mn_tiles < main_tiles ? &map_w : &map_wt;
+    for (; w_ahead < kStages && tl.kb0 + static_cast<int>(w_ahead) < tl.kb1; ++w_ahead) {
+      if (rank == 0) mbar_arrive_expect_tx(&full[w_ahead], 2 * (kABytes + (tl.width / 2) * kBK * 2));
+      tma_load_2d_pair(smem + w_ahead * kStageBytes + kABytes, mw, (tl.kb0 + w_ahead) * kBK,
+                       tl.n0 + rank * (tl.width / 2), &full[w_ahead]);
+    }
+  }
+  RT_PDL_WAIT();  // operands and the output buffer belong to the previous kernel until here
+  const uint32_t tmem_base = *tmem_slot;
+  AbortCtx ab{cta_abort, error_flag};
+
   if (warp == 0) {
     // ------------------------------------------------------------- TMA producer (both CTAs)
     if (lane == 0) {
@@ -136,9 +147,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
           const uint32_t ph = (it / kStages) & 1;
           if (!mbar_wait(&empty[s], ph ^ 1, ab, 111)) { ok = false; break; }
           uint8_t* sa = smem + s * kStageBytes;
-          if (rank == 0) mbar_arrive_expect_tx(&full[s], bytes);
+          if (rank == 0 && it >= w_ahead) mbar_arrive_expect_tx(&full[s], bytes);
           tma_load_2d_pair(sa, &map_a, kb * kBK, m0, &full[s]);
-          tma_load_2d_pair(sa + kABytes, mw, kb * kBK, n0, &full[s]);
+          if (it >= w_ahead) tma_load_2d_pair(sa + kABytes, mw, kb * kBK, n0, &full[s]);
         }
       }
     }
@@ -247,8 +258,12 @@ rt_status launch_pair(void* c, const void* a, const void* w, const void* bias, i
   const int mn = main_tiles + ((M + kTileM - 1) / kTileM) * (N / tail_w) - (main_tiles ? main_tiles * (kTileN / tail_w) : 0);
   const int tiles = mn * (EPI == kEpiPartial ? qkv.splits : 1);
   const int pairs = std::min(tiles, sms / 2);
+  // Only where the launch fills the chip.  12 layers: 4096 tokens 1177 -> 1173 us, 5312 1279 -> 1272, 1024 wide (24 layers) 4096
+  // tokens 3462 -> 3421; with CTAs that wait on free SMs for longer, 256 tokens 435 -> 437, 1024 wide 1024 tokens 1544 -> 1550.
+  QkvEpilogue args = qkv;
+  args.settled_w = qkv.settled_w && pairs == sms / 2;
   RT_CHECK_CUDA(launch_kernel(kern, dim3(2 * pairs), dim3(kThreads), kSmemBytes, st, ma, mw, mwt, mc, mk, mv, main_tiles, tail_w, (uint16_t*)c,
-                              (const uint16_t*)bias, M, N, K, err, qkv));
+                              (const uint16_t*)bias, M, N, K, err, args));
   count_launch();
   RT_CHECK_CUDA(cudaGetLastError());
   return RT_OK;

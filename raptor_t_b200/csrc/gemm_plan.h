@@ -21,7 +21,10 @@ GemmPlan plan_gemm(int M, int N, int K, int max_splits, bool parts);
 rt_status run_gemm(void* c, const void* a, const void* w, const void* bias, int M, int N, int K, int epi, int dtype,
                    cudaStream_t st, const gemm_detail::QkvEpilogue& extra, const GemmPlan& plan);
 
-// rt_gemm and rt_gemm_qkv; settled_w as in QkvEpilogue.
+// rt_gemm, rt_gemm_bias_residual_layernorm and rt_gemm_qkv; settled_w as in QkvEpilogue.
+rt_status gemm_layernorm_checked(void* out, const void* a, const void* w, const void* bias, const void* residual,
+                                 const void* gamma, const void* beta, int M, int N, int K, float eps, int dtype,
+                                 void* stream, bool settled_w);
 rt_status gemm_checked(void* c, const void* a, const void* w, const void* bias, int M, int N, int K, int epilogue,
                        int dtype, void* stream, const gemm_detail::QkvEpilogue& extra);
 rt_status gemm_qkv_checked(void* q, void* k, void* v, const void* a, const void* w, const void* bias,
