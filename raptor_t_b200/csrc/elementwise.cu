@@ -240,6 +240,74 @@ __global__ void __launch_bounds__(1024) layernorm_parts_kernel(T* __restrict__ o
 }
 
 // ---------------------------------------------------------------------------
+// The same with one warp per row, four columns of every 128 per lane: all loads of a part, or of two, are in flight
+// together and nothing but shuffles joins a row.  Against one CTA per row, us alone: 320 x 768, four parts 3.6 -> 2.7, 512, three
+// parts 3.7 -> 2.7, 2048, two 5.0 -> 3.3, 6144, one 11.2 -> 5.1 (L2: 9.6 TB/s).
+// ---------------------------------------------------------------------------
+constexpr int kPartsThreads = 128;
+template <typename T, int NV>
+__global__ void __launch_bounds__(kPartsThreads, 4)
+layernorm_parts_rows_kernel(T* __restrict__ out, const float* __restrict__ parts, const T* __restrict__ bias,
+                            const T* __restrict__ residual, const T* __restrict__ gamma, const T* __restrict__ beta, int rows,
+                       int splits, float eps) {
+  constexpr int kHidden = NV * 128;
+  constexpr int kWarps = kPartsThreads / 32;
+  RT_PDL_LAUNCH_DEPENDENTS();
+  const int col = (threadIdx.x & 31) * 4;
+  const size_t stride = static_cast<size_t>(rows) * kHidden;
+  RT_PDL_WAIT();
+  for (int row = blockIdx.x * kWarps + (threadIdx.x >> 5); row < rows; row += gridDim.x * kWarps) {
+    const size_t at = static_cast<size_t>(row) * kHidden + col;
+    uint2 res[NV];
+    float v[NV][4];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      res[i] = *reinterpret_cast<const uint2*>(residual + at + i * 128);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) v[i][k] = 0.f;
+    }
+#pragma unroll 2
+    for (int s = 0; s < splits; ++s)
+#pragma unroll
+      for (int i = 0; i < NV; ++i) {
+        const float4 p = *reinterpret_cast<const float4*>(parts + s * stride + at + i * 128);
+        v[i][0] += p.x;
+        v[i][1] += p.y;
+        v[i][2] += p.z;
+        v[i][3] += p.w;
+      }
+    float sum = 0.f;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      float bb[4], rr[8];
+      unpack4(bias + col + i * 128, bb);
+      Vec8<T>::unpack(make_uint4(res[i].x, res[i].y, 0u, 0u), rr);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        v[i][k] += bb[k] + rr[k];
+        sum += v[i][k];
+      }
+    }
+    const float mean = warp_sum(sum) * (1.0f / kHidden);
+    float sq = 0.f;
+#pragma unroll
+    for (int i = 0; i < NV; ++i)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) sq += (v[i][k] - mean) * (v[i][k] - mean);
+    const float rstd = rsqrtf(warp_sum(sq) * (1.0f / kHidden) + eps);
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      float gg[4], be[4], o[4];
+      unpack4(gamma + col + i * 128, gg);
+      unpack4(beta + col + i * 128, be);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) o[k] = (v[i][k] - mean) * rstd * gg[k] + be[k];
+      pack4(o, out + at + i * 128);
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
 // bias + GELU (tanh form), in place, one 128-bit vector per thread per step.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ float gelu_tanh(float x) {
@@ -465,21 +533,55 @@ static rt_status layernorm_launch(void* out, const void* x, const void* bias, co
   return RT_OK;
 }
 
-// out = LayerNorm(sum of the parts + bias + residual) * gamma + beta; hidden % 128 == 0, hidden <= 4096
+template <typename T>
+static rt_status layernorm_parts_launch(T* out, const float* parts, int splits, const T* bias, const T* residual,
+                                        const T* gamma, const T* beta, int rows, int hidden, float eps, cudaStream_t st) {
+  // In the chain of a forward (12 layers, us, one CTA / one warp per row): 320 tokens 486 / 479, 640 584 / 581, 832 630 / 627,
+  // 1728 841 / 828, 1984 879 / 863, 6144 1678 / 1633; but 128 tokens 373 / 377, 1024 674 / 678, 1472 807.8 / 809, and 1024
+  // wide 320 tokens 1132 / 1142, 896 1513 / 1571: there the many small CTAs leave the next GEMM's start alone.
+  const bool warp_per_row = rows >= 1536 || (hidden <= 768 && rows > 256 && rows < 960);
+  if (!warp_per_row) {
+    RT_CHECK_CUDA(launch_kernel(layernorm_parts_kernel<T>, dim3(rows), dim3(hidden / 4), 0, st, out, parts, bias, residual,
+                                gamma, beta, rows, hidden, splits, eps));
+    count_launch();
+    RT_CHECK_CUDA(cudaGetLastError());
+    return RT_OK;
+  }
+  const int per_cta = kPartsThreads / 32;
+  const int blocks = std::min((rows + per_cta - 1) / per_cta, 4 * sm_count());
+#define RT_PARTS_CASE(NV)                                                                                            \
+  case NV:                                                                                                           \
+    RT_CHECK_CUDA(launch_kernel(layernorm_parts_rows_kernel<T, NV>, dim3(blocks), dim3(kPartsThreads), 0, st, out, parts, \
+                                bias, residual, gamma, beta, rows, splits, eps));                                    \
+    break;
+  switch (hidden / 128) {
+    RT_PARTS_CASE(1)
+    RT_PARTS_CASE(2)
+    RT_PARTS_CASE(3)
+    RT_PARTS_CASE(4)
+    RT_PARTS_CASE(5)
+    RT_PARTS_CASE(6)
+    RT_PARTS_CASE(7)
+    RT_PARTS_CASE(8)
+    default:
+      return fail(RT_ERR_UNSUPPORTED, "layernorm_parts: hidden=%d not supported", hidden);
+  }
+#undef RT_PARTS_CASE
+  count_launch();
+  RT_CHECK_CUDA(cudaGetLastError());
+  return RT_OK;
+}
+
+// out = LayerNorm(sum of the parts + bias + residual) * gamma + beta; hidden % 128 == 0, hidden <= 1024
 rt_status layernorm_parts(void* out, const float* parts, int splits, const void* bias, const void* residual,
                           const void* gamma, const void* beta, int rows, int hidden, float eps, int dtype,
                           cudaStream_t st) {
   if (dtype == RT_BF16)
-    RT_CHECK_CUDA(launch_kernel(layernorm_parts_kernel<__nv_bfloat16>, dim3(rows), dim3(hidden / 4), 0, st,
-                                (__nv_bfloat16*)out, parts, (const __nv_bfloat16*)bias, (const __nv_bfloat16*)residual,
-                                (const __nv_bfloat16*)gamma, (const __nv_bfloat16*)beta, rows, hidden, splits, eps));
-  else
-    RT_CHECK_CUDA(launch_kernel(layernorm_parts_kernel<__half>, dim3(rows), dim3(hidden / 4), 0, st, (__half*)out, parts,
-                                (const __half*)bias, (const __half*)residual, (const __half*)gamma, (const __half*)beta,
-                                rows, hidden, splits, eps));
-  count_launch();
-  RT_CHECK_CUDA(cudaGetLastError());
-  return RT_OK;
+    return layernorm_parts_launch((__nv_bfloat16*)out, parts, splits, (const __nv_bfloat16*)bias,
+                                  (const __nv_bfloat16*)residual, (const __nv_bfloat16*)gamma, (const __nv_bfloat16*)beta,
+                                  rows, hidden, eps, st);
+  return layernorm_parts_launch((__half*)out, parts, splits, (const __half*)bias, (const __half*)residual,
+                                (const __half*)gamma, (const __half*)beta, rows, hidden, eps, st);
 }
 
 }  // namespace rt
