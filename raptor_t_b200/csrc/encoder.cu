@@ -441,9 +441,11 @@ rt_status ensure_scratch(rt_encoder* e, int tokens) {
 // FFN down + LayerNorm for batches of few tokens: split-K GEMM into fp32 parts and a LayerNorm that sums them.
 // The cluster kernel walks all K blocks of a row block in sequence, however few row blocks there are (K = 3072:
 // 17.1 us for 128 rows, 17.4 for 1024, 17.9 for 2048, 19.1 for 4096); cut along K until the chip is full, projection
-// and LayerNorm take 10.9 for 512 rows, 12.3 for 1024, 17.6 for 2048; up to 256 rows the split is one over a cluster
-// (plan_gemm), whose sums are one part (256 rows 10.1 -> 8.9 us, 1024 wide 11.1 -> 10.1).  Estimates in microseconds, as in plan_gemm
-// (both sides a little high: the line between them lies at 2048 rows).  With K = 768 or 1024 the parts' traffic eats
+// and LayerNorm take 10.6 for 512 rows, 12.3 for 1024, 16.8 for 2048, 16.9 for 2304 (cluster kernel 19.6), 20.1 for 2560
+// (19.5); up to 256 rows the split is one over a cluster (plan_gemm), whose sums are one part (256 rows 10.1 -> 8.9 us,
+// 1024 wide 11.1 -> 10.1).  Estimates in microseconds, as in plan_gemm, both sides a little high: a launch of the
+// LayerNorm counts 2.5, 1.5 where one warp takes a row (layernorm_parts), which sets the 768-wide line at 2304 rows as
+// measured (12 layers: 2112 tokens 906 -> 862 us, 2304 913 -> 868).  With K = 768 or 1024 the parts' traffic eats
 // the gain (8.0 against 6.9 us for 128 rows): not used.
 bool plan_parts(const rt_encoder* e, int K, GemmPlan& plan) {
   const int M = e->tokens, N = e->cfg.hidden;
@@ -454,7 +456,7 @@ bool plan_parts(const rt_encoder* e, int K, GemmPlan& plan) {
   plan = plan_gemm(M, N, K, max_splits, true);
   if (plan.cluster) return true;  // one part
   const double rows = static_cast<double>(M) * N;
-  const double parts_cost = plan.cost + 2.5 + rows * 6 / 6e6;
+  const double parts_cost = plan.cost + (M >= 1536 ? 1.5 : 2.5) + rows * 6 / 6e6;
   double other;
   if (N == 768) {  // LayerNorm is part of the cluster kernel's epilogue; 36 clusters of 128 rows, 22 of 256 are resident
     if (M <= 36 * 128) other = 7.2 + K / 64 * 0.21 + M * 0.0007;

@@ -19,7 +19,7 @@ def test_ffn_down_of_small_batches(hidden, dtype):
     pre = "encoder.layer.0.output."
     W = {k: P[pre + k].cuda().to(td).double() for k in ("dense.weight", "dense.bias", "LayerNorm.weight", "LayerNorm.bias")}
     split = 0
-    for rows in (64, 256, 320, 896, 960, 1024, 1472, 1536, 1600, 2048, 5888, 6144):
+    for rows in (64, 256, 320, 896, 960, 1024, 1472, 1536, 1600, 2048, 2112, 2304, 2368, 5888, 6144):
         enc.prepare([rows] if rows <= 4096 and rows != 768 else [rows // 2] * 2)
         split += enc.get_option("ffn_down_parts") > 0
         gen = torch.Generator(device="cuda").manual_seed(rows)
