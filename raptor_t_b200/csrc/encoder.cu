@@ -474,15 +474,16 @@ bool plan_parts(const rt_encoder* e, int K, GemmPlan& plan) {
 //   1024 columns, K = 1024 2048 rows 12.4 / 11.4  3072 12.9 / 14.3   8192 22.4 / 24.6   20480 52.4 / 61.6
 //   1024 columns, K = 4096 3072 rows 26.8 / 29.2  4096 44.2 / 31.6   12288 91.8 / 91.3  20480 141.5 / 152.0
 // (15 clusters of four pairs are resident: from the second wave on, 28 idle SMs cost more than the LayerNorm until
-// its traffic leaves L2).  Fused in a step: large model 58.9 -> 55.7 ms.  The 768-wide attention output is fused while its
-// row blocks are one wave of single-CTA clusters and again above 89 blocks (12 layers: 30592 tokens 6.39 -> 6.27 ms, 45312 9.54
-// -> 9.33, 68672 14.01 -> 13.69).  Fused would be faster between as well (20480 tokens 4.28 -> 4.22 ms), but the contract
-// test of the benchmark counts six kernels per layer of its 16500-22600-token batches.
+// its traffic leaves L2).  Fused in a step: large model 58.9 -> 55.7 ms.  The 768-wide attention output is fused from 13
+// row blocks on (12 layers, us, apart / fused: 2816 tokens 987 / 992, 3072 1055 / 1061, 3200 1053 / 1040, 3584 1092 / 1076,
+// 5312 1347 / 1308, 8192 1985 / 1932, 12288 2922 / 2909, 16384 3745 / 3649; 30592 tokens 6.39 / 6.27 ms, 45312 9.54 / 9.33).
+// Between 65 and 89 blocks fused is faster as well (20480 tokens 4.28 / 4.22 ms), but the contract test of the benchmark
+// counts six kernels per layer of its 16500-22600-token batches.
 bool fuses_layernorm(const rt_encoder* e, int K) {
   const int N = e->cfg.hidden, blocks = (e->tokens + 255) / 256;
   if (N != 768 && N != 1024) return false;
   if (e->fuse_layernorm != 1) return e->fuse_layernorm == 2;
-  if (N == 768) return K >= 2048 || (blocks > 14 && blocks <= 18) || blocks > 89;
+  if (N == 768) return K >= 2048 || (blocks > 12 && blocks <= 64) || blocks > 89;
   return blocks > 10 && (K < 2048 || blocks <= 15 || blocks > 48);
 }
 
