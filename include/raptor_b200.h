@@ -249,8 +249,8 @@ rt_status rt_encoder_set_embeddings(rt_encoder* enc, const void* word, const voi
                                     const void* ln_g, const void* ln_b);
 
 /* Per-batch metadata: varlen offsets, block tables and attention work lists of every layer are
- * built by a host worker thread and uploaded on a side stream, one event per layer; the
- * forward pass waits on layer i's event right before layer i's attention kernel.
+ * built by a host worker thread and uploaded on a side stream, one event per upload; the
+ * forward pass waits for layer i's right before layer i's attention kernel.
  * layers/metadata.cpp:6-18 (MetaData::update_meta_data) + layers/semaphore.cpp:16-37 +
  * layers/tensor_set.cpp:10-25 (scratch resize). */
 rt_status rt_encoder_prepare_batch(rt_encoder* enc, const int32_t* lens_tokens, int n_seq);
