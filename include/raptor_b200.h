@@ -239,7 +239,9 @@ rt_status rt_encoder_destroy(rt_encoder* enc);
 /* Weights of one layer, 16-bit device pointers, copied into the object (re-laid-out once).
  * qkv_w [hidden][3*hidden] and the other matrices are [in][out] exactly as the reference's
  * Python wrappers pass them (python/modeling_bert.py:138-163, 84-91, 107-113);
- * in_out_layout = 0 means the torch Linear layout [out][in] instead. */
+ * in_out_layout = 0 means the torch Linear layout [out][in] instead.  This call and
+ * rt_encoder_set_embeddings wait for the device before and after their copies: forwards issued
+ * earlier finish with the old parameters, later ones on any stream have the new ones. */
 rt_status rt_encoder_set_layer(rt_encoder* enc, int layer, uint32_t table_seed, int in_out_layout,
                                const void* qkv_w, const void* qkv_b, const void* attn_out_w,
                                const void* attn_out_b, const void* attn_ln_g, const void* attn_ln_b,

@@ -245,7 +245,6 @@ rt_status copy_or_transpose(DevBuf& dst, const void* src, int rows_in, int cols_
     dim3 grid((cols_in + 31) / 32, (rows_in + 31) / 32), block(32, 8);
     transpose16_kernel<<<grid, block>>>((uint16_t*)dst.p, (const uint16_t*)src, rows_in, cols_in);
     RT_CHECK_CUDA(cudaGetLastError());
-    RT_CHECK_CUDA(cudaDeviceSynchronize());
   }
   return RT_OK;
 }
@@ -253,6 +252,19 @@ rt_status copy_or_transpose(DevBuf& dst, const void* src, int rows_in, int cols_
 rt_status copy_vec(DevBuf& dst, const void* src, size_t bytes) {
   RT_TRY(dst.ensure(bytes));
   RT_CHECK_CUDA(cudaMemcpy(dst.p, src, bytes, cudaMemcpyDeviceToDevice));
+  return RT_OK;
+}
+
+// Parameters are replaced while the device is idle: forwards on streams that the copies' stream is not ordered with may
+// still read the old ones, and later ones, whose GEMMs request weights ahead of the kernels before them
+// (QkvEpilogue::settled_w), must find the new ones in place: copies within the device return before they have ended.
+rt_status set_parameters_begin(rt_encoder* e) {
+  e->join_worker();
+  RT_CHECK_CUDA(cudaDeviceSynchronize());
+  return RT_OK;
+}
+rt_status set_parameters_end() {
+  RT_CHECK_CUDA(cudaDeviceSynchronize());
   return RT_OK;
 }
 
@@ -498,7 +510,7 @@ bool aligned(size_t bytes, std::initializer_list<const void*> ptrs) {
 }
 bool always_fused(const rt_encoder* e, int K) { return e->fuse_layernorm == 2 || (e->cfg.hidden == 768 && K >= 2048); }
 
-// The encoder's weights are written by rt_encoder_set_layer alone, never by a kernel that a forward's may overlap.
+// The encoder's weights are written by rt_encoder_set_layer alone, while the device is idle.
 gemm_detail::QkvEpilogue weights_settled() {
   gemm_detail::QkvEpilogue extra{};
   extra.settled_w = true;
@@ -751,7 +763,7 @@ extern "C" rt_status rt_encoder_set_layer(rt_encoder* e, int layer, uint32_t tab
   RT_REQUIRE(layer >= 0 && layer < e->cfg.layers, RT_ERR_INVALID, "set_layer: layer %d out of range", layer);
   RT_REQUIRE(qkv_w && qkv_b && ao_w && ao_b && aln_g && aln_b && up_w && up_b && down_w && down_b && oln_g && oln_b,
              RT_ERR_INVALID, "set_layer: null weight pointer");
-  e->join_worker();
+  RT_TRY(set_parameters_begin(e));
   const int H = e->cfg.hidden, F = e->cfg.ffn;
   LayerWeights& w = e->layers[layer];
   const bool tr = in_out_layout != 0;
@@ -768,6 +780,7 @@ extern "C" rt_status rt_encoder_set_layer(rt_encoder* e, int layer, uint32_t tab
   RT_TRY(copy_vec(w.down_b, down_b, H * elt()));
   RT_TRY(copy_vec(w.oln_g, oln_g, H * elt()));
   RT_TRY(copy_vec(w.oln_b, oln_b, H * elt()));
+  RT_TRY(set_parameters_end());
   w.seed = table_seed;
   w.set = true;
   return RT_OK;
@@ -777,11 +790,13 @@ extern "C" rt_status rt_encoder_set_embeddings(rt_encoder* e, const void* word, 
                                                const void* ln_g, const void* ln_b) {
   RT_REQUIRE(e && word && pos && type && ln_g && ln_b, RT_ERR_INVALID, "set_embeddings: null pointer");
   const size_t H = e->cfg.hidden;
+  RT_TRY(set_parameters_begin(e));
   RT_TRY(copy_vec(e->emb_word, word, static_cast<size_t>(e->cfg.vocab) * H * 4));
   RT_TRY(copy_vec(e->emb_pos, pos, static_cast<size_t>(e->cfg.max_pos) * H * 4));
   RT_TRY(copy_vec(e->emb_type, type, static_cast<size_t>(e->cfg.type_vocab) * H * 4));
   RT_TRY(copy_vec(e->emb_g, ln_g, H * 4));
   RT_TRY(copy_vec(e->emb_b, ln_b, H * 4));
+  RT_TRY(set_parameters_end());
   e->emb_set = true;
   return RT_OK;
 }
