@@ -485,18 +485,16 @@ bool plan_parts(const rt_encoder* e, int K, GemmPlan& plan) {
 //   768 columns, K = 3072  4096 rows 20.2 / 20.2  8192 36.0 / 36.1   20480 81.8 / 93.3
 //   1024 columns, K = 1024 2048 rows 12.4 / 11.4  3072 12.9 / 14.3   8192 22.4 / 24.6   20480 52.4 / 61.6
 //   1024 columns, K = 4096 3072 rows 26.8 / 29.2  4096 44.2 / 31.6   12288 91.8 / 91.3  20480 141.5 / 152.0
-// (15 clusters of four pairs are resident, so 28 SMs idle: from the second wave on that costs more than the LayerNorm until
-// its traffic leaves L2, unless the projection alone needs as many waves of its 74 pairs; 24 layers, apart / fused: 4096 tokens
-// 3315 / 3499, 4864 4028 / 4005, 7168 5525 / 5387, 8192 6078 / 6221, 9216 6733 / 6855, 10240 7494 / 7380, 11008 7991 / 7849).  Fused in a step: large model 58.9 -> 55.7 ms.  The 768-wide attention output is fused from 13
-// row blocks on (12 layers, us, apart / fused: 2816 tokens 987 / 992, 3072 1055 / 1061, 3200 1053 / 1040, 3584 1092 / 1076,
-// 5312 1347 / 1308, 8192 1985 / 1932, 12288 2922 / 2909, 16384 3745 / 3649; 30592 tokens 6.39 / 6.27 ms, 45312 9.54 / 9.33).
-// Between 65 and 89 blocks fused is faster as well (20480 tokens 4.28 / 4.22 ms), but the contract test of the benchmark
-// counts six kernels per layer of its 16500-22600-token batches.
+// 768-wide attention output, 12 layers, us, apart / fused: 3072 tokens 1055 / 1061, 3200 1053 / 1040, 5312 1347 / 1308,
+// 16384 3745 / 3649, 16512 3806 / 3712, 20352 4646 / 4596, 22656 5262 / 5177, 45312 9540 / 9330.
+// 1024-wide FFN down: 15 clusters of four pairs are resident, so 28 SMs idle.  From the second wave on that costs more than
+// the LayerNorm until its traffic leaves L2, unless the projection alone needs as many waves of its 74 pairs (24 layers,
+// apart / fused: 4096 tokens 3315 / 3499, 4864 4028 / 4005, 8192 6078 / 6221, 10240 7494 / 7380, 11008 7991 / 7849).
 bool fuses_layernorm(const rt_encoder* e, int K) {
   const int N = e->cfg.hidden, blocks = (e->tokens + 255) / 256;
   if (N != 768 && N != 1024) return false;
   if (e->fuse_layernorm != 1) return e->fuse_layernorm == 2;
-  if (N == 768) return K >= 2048 || (blocks > 12 && blocks <= 64) || blocks > 89;
+  if (N == 768) return K >= 2048 || blocks > 12;
   return blocks > 10 && (K < 2048 || blocks > 48 || (blocks + 14) / 15 <= (blocks * 4 + 73) / 74);
 }
 
