@@ -187,9 +187,8 @@ layernorm_kernel(T* __restrict__ out, const T* __restrict__ x, const T* __restri
 
 // ---------------------------------------------------------------------------
 // The same over a projection given as `splits` fp32 parts [splits][rows][hidden] (split-K GEMM): sums the
-// parts, adds bias and residual, normalises.  One CTA per row, four columns per thread: used for batches of
-// few rows, where the latency of the part loads bounds it (all parts of a row are in flight together) and one
-// warp per row would leave most SMs without work.
+// parts, adds bias and residual, normalises.  One CTA per row, four columns per thread: bound by the latency of the
+// part loads (all parts of a row are in flight together).
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ float block_sum(float v, float* s_warp) {
   v = warp_sum(v);
@@ -241,8 +240,8 @@ __global__ void __launch_bounds__(1024) layernorm_parts_kernel(T* __restrict__ o
 
 // ---------------------------------------------------------------------------
 // The same with one warp per row, four columns of every 128 per lane: all loads of a part, or of two, are in flight
-// together and nothing but shuffles joins a row.  Against one CTA per row, us alone: 320 x 768, four parts 3.6 -> 2.7, 512, three
-// parts 3.7 -> 2.7, 2048, two 5.0 -> 3.3, 6144, one 11.2 -> 5.1 (L2: 9.6 TB/s).
+// together and nothing but shuffles joins a row.  Against one CTA per row, us alone: 320 x 768, four parts 3.6 -> 2.7,
+// 512, three parts 3.7 -> 2.7, 2048, two 5.0 -> 3.3, 6144, one 11.2 -> 5.1 (37.7 MB: 7.4 TB/s, out of L2).
 // ---------------------------------------------------------------------------
 constexpr int kPartsThreads = 128;
 template <typename T, int NV>
@@ -533,14 +532,21 @@ static rt_status layernorm_launch(void* out, const void* x, const void* bias, co
   return RT_OK;
 }
 
+// One warp per row or one CTA.  12 layers, us, one CTA / one warp per row, 20 to 30 repeats in turn:
+//   512 columns  320 rows 421.9 / 417.1   640 486.8 / 480.6   1024 517.3 / 505.9   1600 587.8 / 579.7
+//   640 columns  320 rows 452.1 / 444.4   640 533.9 / 523.6   1152 587.1 / 587.1   1792 647.1 / 630.2
+//   768 columns  320 rows 487.4 / 478.7   512 542.0 / 538.7   576 550.0 / 556.2    704 567.4 / 575.5
+//                1024 604.3 / 608.3       1472 670.9 / 671.7  1536 685.2 / 672.9   2304 793.8 / 772.1   6144 1420 / 1359
+// Up to 256 rows neither is faster (768 columns 128 rows 376.2 / 380.2); 1024 columns (up to 1152 rows) are slower with
+// warps, 512 rows 624.6 / 634.2, 1024 741.2 / 768.0, 896 equal: there the many small CTAs leave the next GEMM's start alone.
+bool layernorm_parts_by_warps(int rows, int hidden) {
+  return rows > 256 && (hidden <= 640 || (hidden <= 768 && (rows <= 512 || rows >= 1536)));
+}
+
 template <typename T>
 static rt_status layernorm_parts_launch(T* out, const float* parts, int splits, const T* bias, const T* residual,
                                         const T* gamma, const T* beta, int rows, int hidden, float eps, cudaStream_t st) {
-  // In the chain of a forward (12 layers, us, one CTA / one warp per row): 320 tokens 486 / 479, 640 584 / 581, 832 630 / 627,
-  // 1728 841 / 828, 1984 879 / 863, 6144 1678 / 1633; but 128 tokens 373 / 377, 1024 674 / 678, 1472 807.8 / 809, and 1024
-  // wide 320 tokens 1132 / 1142, 896 1513 / 1571: there the many small CTAs leave the next GEMM's start alone.
-  const bool warp_per_row = rows >= 1536 || (hidden <= 768 && rows > 256 && rows < 960);
-  if (!warp_per_row) {
+  if (!layernorm_parts_by_warps(rows, hidden)) {
     RT_CHECK_CUDA(launch_kernel(layernorm_parts_kernel<T>, dim3(rows), dim3(hidden / 4), 0, st, out, parts, bias, residual,
                                 gamma, beta, rows, hidden, splits, eps));
     count_launch();
@@ -561,8 +567,6 @@ static rt_status layernorm_parts_launch(T* out, const float* parts, int splits, 
     RT_PARTS_CASE(4)
     RT_PARTS_CASE(5)
     RT_PARTS_CASE(6)
-    RT_PARTS_CASE(7)
-    RT_PARTS_CASE(8)
     default:
       return fail(RT_ERR_UNSUPPORTED, "layernorm_parts: hidden=%d not supported", hidden);
   }
@@ -576,6 +580,8 @@ static rt_status layernorm_parts_launch(T* out, const float* parts, int splits, 
 rt_status layernorm_parts(void* out, const float* parts, int splits, const void* bias, const void* residual,
                           const void* gamma, const void* beta, int rows, int hidden, float eps, int dtype,
                           cudaStream_t st) {
+  RT_REQUIRE(hidden > 0 && hidden % 128 == 0 && hidden <= 1024, RT_ERR_UNSUPPORTED, "layernorm_parts: hidden=%d not supported",
+             hidden);
   if (dtype == RT_BF16)
     return layernorm_parts_launch((__nv_bfloat16*)out, parts, splits, (const __nv_bfloat16*)bias,
                                   (const __nv_bfloat16*)residual, (const __nv_bfloat16*)gamma, (const __nv_bfloat16*)beta,

@@ -120,6 +120,7 @@ namespace rt {
 rt_status layernorm_parts(void* out, const float* parts, int splits, const void* bias, const void* residual,
                           const void* gamma, const void* beta, int rows, int hidden, float eps, int dtype,
                           cudaStream_t st);  // elementwise.cu
+bool layernorm_parts_by_warps(int rows, int hidden);
 }
 
 using namespace rt;
@@ -456,19 +457,19 @@ rt_status ensure_scratch(rt_encoder* e, int tokens) {
 // and LayerNorm take 10.6 for 512 rows, 12.3 for 1024, 16.8 for 2048, 16.9 for 2304 (cluster kernel 19.6), 20.1 for 2560
 // (19.5); up to 256 rows the split is one over a cluster (plan_gemm), whose sums are one part (256 rows 10.1 -> 8.9 us,
 // 1024 wide 11.1 -> 10.1).  Estimates in microseconds, as in plan_gemm, both sides a little high: a launch of the
-// LayerNorm counts 2.5, 1.5 where one warp takes a row (layernorm_parts), which sets the 768-wide line at 2304 rows as
+// LayerNorm counts 2.5, 1.5 where one warp takes a row, which sets the 768-wide line at 2304 rows as
 // measured (12 layers: 2112 tokens 906 -> 862 us, 2304 913 -> 868).  With K = 768 or 1024 the parts' traffic eats
 // the gain (8.0 against 6.9 us for 128 rows): not used.
 bool plan_parts(const rt_encoder* e, int K, GemmPlan& plan) {
   const int M = e->tokens, N = e->cfg.hidden;
-  if (M == 0 || e->fuse_layernorm != 1 || e->fuse_residual || K < 2048 || N % 128 != 0 || N > 4096) return false;
+  if (M == 0 || e->fuse_layernorm != 1 || e->fuse_residual || K < 2048 || N % 128 != 0 || N > 1024) return false;
   const size_t part = static_cast<size_t>(M) * N * 4;
   const int max_splits = static_cast<int>(std::min<size_t>(kLnPartsBytes / part, kMaxLnSplits));
   if (max_splits < 1) return false;
   plan = plan_gemm(M, N, K, max_splits, true);
   if (plan.cluster) return true;  // one part
   const double rows = static_cast<double>(M) * N;
-  const double parts_cost = plan.cost + (M >= 1536 ? 1.5 : 2.5) + rows * 6 / 6e6;
+  const double parts_cost = plan.cost + (layernorm_parts_by_warps(M, N) ? 1.5 : 2.5) + rows * 6 / 6e6;
   double other;
   if (N == 768) {  // LayerNorm is part of the cluster kernel's epilogue; 36 clusters of 128 rows, 22 of 256 are resident
     if (M <= 36 * 128) other = 7.2 + K / 64 * 0.21 + M * 0.0007;

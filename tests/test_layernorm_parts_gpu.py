@@ -8,22 +8,24 @@ import oracle
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("hidden,dtype", [(512, "f16"), (768, "f16"), (768, "bf16"), (1024, "bf16")])
+@pytest.mark.parametrize("hidden,dtype", [(128, "bf16"), (256, "f16"), (384, "bf16"), (512, "f16"), (640, "bf16"), (768, "f16"),
+                                          (768, "bf16"), (896, "f16"), (1024, "bf16")])
 def test_ffn_down_of_small_batches(hidden, dtype):
     from raptor_t_b200 import capi, ops
     from raptor_t_b200.engine import Encoder
-    cfg = dict(hidden=hidden, heads=hidden // 64, ffn=4 * hidden, layers=1, max_pos=4096, vocab=97)
+    ffn = max(4 * hidden, 2048)  # shorter sums are not split
+    cfg = dict(hidden=hidden, heads=hidden // 64, ffn=ffn, layers=1, max_pos=4096, vocab=97)
     P = oracle.make_weights(oracle.EncoderConfig(**cfg), seed=5, nonzero_bias=True)
     enc = Encoder(capi.make_config(dtype=dtype, **cfg)).load_weights(P)
     td = torch.float16 if dtype == "f16" else torch.bfloat16
     pre = "encoder.layer.0.output."
     W = {k: P[pre + k].cuda().to(td).double() for k in ("dense.weight", "dense.bias", "LayerNorm.weight", "LayerNorm.bias")}
     split = 0
-    for rows in (64, 256, 320, 896, 960, 1024, 1472, 1536, 1600, 2048, 2112, 2304, 2368, 5888, 6144):
+    for rows in (64, 256, 320, 512, 576, 896, 960, 1024, 1472, 1536, 1600, 2048, 2112, 2304, 2368, 5888, 6144):
         enc.prepare([rows] if rows <= 4096 and rows != 768 else [rows // 2] * 2)
         split += enc.get_option("ffn_down_parts") > 0
         gen = torch.Generator(device="cuda").manual_seed(rows)
-        f = torch.randn(rows, 4 * hidden, device="cuda", generator=gen).to(td)
+        f = torch.randn(rows, ffn, device="cuda", generator=gen).to(td)
         x = torch.randn(rows, hidden, device="cuda", generator=gen).to(td)
         out = enc.output(0, f, x, torch.empty_like(x))
         want = torch.nn.functional.layer_norm(f.double() @ W["dense.weight"].t() + W["dense.bias"] + x.double(), (hidden,),
