@@ -292,14 +292,20 @@ GemmPlan plan_gemm(int M, int N, int K, int max_splits, bool to_parts) {
       consider(kPairTiles[2].at(full, kbs) + c.at(waves(rest * (256 / c.width), pairs), kbs), true, full * pairs, c.width);
   }
   // Two rows of tiles at most and K long enough to be worth sharing: split over clusters, as far as that leaves SMs for
-  // the kernel behind to be resident early (in the chain of a forward, 12 layers: 128 rows 446 -> 381 us, 256 rows
-  // 481 -> 441; with 4 CTAs for each of 36 or 48 tiles 428, for each of the 36 tiles of 384 rows 495 -> 531).  Alone, weights
-  // from HBM, us: 128 rows 768 x 768 5.9 -> 4.8, 3072 x 768 6.3 -> 5.6, 768 x 3072 13.1 -> 5.9, 1024 x 4096 16.4 -> 7.7;
-  // 256 rows 2304 x 768 6.0 -> 5.3, 768 x 3072 13.0 -> 6.8.
-  if (M <= 2 * kBM && K >= 8 * kBK) {
+  // the kernel behind to be resident early.  Not by cost: one launch alone says little about the chain (12 layers, us:
+  // 128 rows 446 -> 381, 256 rows 481 -> 441; with 4 CTAs for each of 36 or 48 tiles 428, for each of the 36 tiles of 384 rows
+  // 495 -> 531).  Alone, weights from HBM, us, tiles / clusters: 128 rows 768 x 768 5.9 / 4.8, 3072 x 768 6.3 / 5.6, 768 x 3072
+  // 13.1 / 5.9, 1024 x 4096 16.4 / 7.7; 256 rows 2304 x 768 6.0 / 5.3, 768 x 3072 13.0 / 6.8.
+  // Left out where the split alone is slower: many pairs of CTAs that read the same few lines of A (columns x K: 64 rows
+  // 4736 x 512 4.51 / 4.86, 4096 x 512 4.54 / 4.68, 4736 x 768 5.40 / 5.57, but 4096 x 768 5.39 / 5.23, 4736 x 1024 6.25 / 5.50;
+  // 32 rows 3072 x 768 5.17 / 5.33, 2560 x 1536 7.63 / 8.37, but 2304 x 768 5.19 / 4.53, 3072 x 3072 12.47 / 8.68), and eight
+  // blocks of K of few rows (32 rows 768 x 512 3.79 / 3.93, 1 row 1536 x 512 3.87 / 4.02, but 32 rows 768 x 640 4.15 / 3.89).
+  if (M <= 2 * kBM && K >= (M < 64 ? 10 : 8) * kBK) {
     const int tiles = mt * (N / kClusterWidth);
     const int cluster = tiles * 8 <= 96 ? 8 : tiles * 4 <= 128 ? 4 : tiles * 2 <= sms ? 2 : 0;
-    if (cluster) best = GemmPlan{false, 0, kClusterWidth, 1, 3.0, cluster};
+    const bool slower = cluster == 2 && ((M < 64 && K < 32 * kBK && tiles > 36) ||
+                                         (M < 96 && K < 16 * kBK && tiles > (K < 12 * kBK ? 56 : 64)));
+    if (cluster && !slower) best = GemmPlan{false, 0, kClusterWidth, 1, 3.0, cluster};
   }
   return best;
 }

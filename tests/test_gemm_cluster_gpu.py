@@ -18,9 +18,11 @@ def _close(got, want, dtype, slack=0.0):
     assert ((got.double() - want).abs() <= rel * want.abs() + 2e-5 + slack).all(), (got.double() - want).abs().max().item()
 
 
-# tiles * 8 <= 96, * 4 <= 128, * 2 <= 148, and one more than that; K blocks that do not divide evenly; rows around a tile's end
-@pytest.mark.parametrize("N", [64, 768, 832, 2048, 2112, 4736, 4800])
-@pytest.mark.parametrize("M,K", [(1, 512), (64, 576), (128, 768), (129, 1024), (191, 3072), (256, 832), (257, 768)])
+# tiles * 8 <= 96, * 4 <= 128, * 2 <= 148, and one more than that; K blocks that do not divide evenly; rows around a tile's end;
+# row blocks filled in part, on both sides of the lines for them
+@pytest.mark.parametrize("N", [64, 768, 832, 2048, 2112, 2304, 2368, 3584, 3648, 4096, 4160, 4736, 4800])
+@pytest.mark.parametrize("M,K", [(1, 512), (48, 640), (32, 2048), (64, 576), (95, 768), (96, 1024), (128, 768), (129, 1024),
+                                 (191, 3072), (256, 832), (257, 768)])
 def test_gemm_of_few_rows(M, N, K):
     from raptor_t_b200 import capi, ops
     dtype = torch.bfloat16 if (M + N // 64) % 2 else torch.float16
