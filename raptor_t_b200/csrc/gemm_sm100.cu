@@ -54,14 +54,16 @@ constexpr int kEpilogueThreads = 256;  // two warps per TMEM lane quarter, alter
 // M = 128 ... 20480 rows of the projections of 768- and 1024-wide models: per launch, per 64-wide K block of a
 // tile, per tile.  A 256-column pair tile does the most work per byte it loads and wins once its waves are full;
 // below that, narrower tiles on more SMs are faster (768 columns, K = 3072, 4096 rows: 48 pair tiles of 256
-// columns 19.9 us, 64 of 192 15.9 us, 192 single-CTA tiles of 128 25.1 us; 1024 columns, K = 4096, one wave of 256
-// columns either way: 2409 rows 27.6 us with single CTAs and 26.8 with pairs, 3840 rows 29.5 and 26.8, 4454 31.0 and 28.8).
+// columns 19.9 us, 64 of 192 15.9 us, 192 single-CTA tiles of 128 25.1 us).  For as many waves of 256 columns the
+// pairs stay ahead: alone, us, single CTAs / pairs, 1024 columns: 3840 rows K = 4096 29.5 / 26.8, 5120 33.1 / 30.9, 8192
+// 54.6 / 49.7, 4454 rows K = 4096 31.0 / 28.8.  Up to K = 2048 single CTAs are faster alone (K = 1024, 3840 rows 9.6 / 10.5) but not in
+// the chain of a forward, where pairs start earlier (12 layers of 1024 columns, 1024 tokens, FFN up 781 / 775, 1536, QKV 930 / 922).
 struct TileCost {
   int width;
   double launch, k_block, tile;
   double at(int waves, int k_blocks) const { return launch + waves * (k_blocks * k_block + tile); }
 };
-constexpr TileCost kSingleTiles[3] = {{64, 2.3, 0.2, 0.45}, {128, 2.6, 0.235, 0.6}, {256, 3.2, 0.286, 2.1}};
+constexpr TileCost kSingleTiles[3] = {{64, 2.3, 0.2, 0.45}, {128, 2.6, 0.235, 0.6}, {256, 3.2, 0.29, 2.1}};
 constexpr TileCost kPairTiles[3] = {{128, 3.6, 0.2, 0.5}, {192, 3.6, 0.24, 1.0}, {256, 3.8, 0.29, 1.2}};
 // the last, partial wave of 256-column pair tiles cut into narrower ones
 constexpr TileCost kTailTiles[2] = {{64, 0, 0.15, 0.5}, {128, 0, 0.2, 0.6}};

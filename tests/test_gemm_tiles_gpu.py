@@ -19,7 +19,7 @@ def _gelu(x):
 @pytest.mark.parametrize("m,n,k", [(1, 768, 768), (129, 768, 3072), (1024, 768, 768), (2047, 768, 768), (4096, 768, 768),
                                    (5003, 768, 768), (8192, 768, 768), (7001, 768, 1024), (1025, 2304, 768),
                                    (2048, 2304, 768), (4353, 2304, 768), (1024, 3072, 768), (2049, 3072, 768),
-                                   (5003, 3072, 768), (20481, 768, 768), (300, 320, 128), (300, 192, 64)])
+                                   (5003, 3072, 768), (20481, 768, 768), (300, 320, 128), (300, 192, 64), (2305, 1024, 5120)])
 @pytest.mark.parametrize("gelu", [False, True])
 def test_gemm_tile_shapes(m, n, k, dtype, gelu):
     from raptor_t_b200 import capi, ops
