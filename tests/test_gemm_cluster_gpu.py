@@ -35,7 +35,10 @@ def test_gemm_of_few_rows(M, N, K):
     gelu = torch.nn.functional.gelu(acc + bias.double(), approximate="tanh")
     _close(ops.gemm(a, w, bias, capi.RT_EPI_BIAS_GELU, out=out[:M]), gelu, dtype,
            2.0 ** -11 * (acc + bias.double()).abs())
+    res = torch.randn(M, N, device="cuda", generator=torch.Generator(device="cuda").manual_seed(7)).to(dtype)
+    _close(ops.gemm_residual(a, w, bias, res, out=out[:M]), acc + bias.double() + res.double(), dtype)
     assert (out[M] == 7.0).all()  # nothing behind the last row
+    assert torch.equal(ops.gemm_residual(a, w, bias, res, out=res), out[:M])  # over the residual
     first = ops.gemm(a, w, bias, capi.RT_EPI_BIAS, out=torch.empty_like(out[:M])).clone()
     assert torch.equal(first, ops.gemm(a, w, bias, capi.RT_EPI_BIAS, out=torch.empty_like(out[:M])))
     ops.check_device()
