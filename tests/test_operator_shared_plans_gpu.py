@@ -52,3 +52,45 @@ def test_models_alive_together_match_the_oracle(lens):
         check(cfg, P, m)
     md.terminate_thread()
     ops.check_device()
+
+
+def test_models_on_two_streams_share_partial_results():
+    """A list that is cut leaves its partial results in the plan, which both models now share: forwards of the two on two
+    streams, issued without any synchronisation, layer by layer in turn, come out as alone."""
+    from raptor_t_b200 import compiled, metadata, ops
+    raptor_t = compiled.load()
+    models = [_model(raptor_t, 2, seed)[2] for seed in (3, 4)]
+    md = raptor_t.MetaData()
+    lens = [4096]
+    prefix, total, _, _ = metadata.generate_data_metainfo(lens, 64, 160, 2)
+    T = sum(lens)
+    gen = torch.Generator(device="cuda").manual_seed(2)
+    x = [torch.randn(T, 128, device="cuda", generator=gen).half() for _ in models]
+    mask = None
+    prefix_dev = torch.tensor(prefix, dtype=torch.int32, device="cuda")
+    md.update_meta_data(T, prefix[-1] + 1, total, prefix)
+
+    def attention(m, layer, src, dst):
+        m.encoder.layer[layer].attention(src, mask, dst, prefix, prefix_dev, None, None, 160, {})
+
+    want = []
+    for m, src in zip(models, x):
+        a, b = torch.empty_like(src), torch.empty_like(src)
+        attention(m, 0, src, a)
+        attention(m, 1, a, b)
+        want.append(b)
+        torch.cuda.synchronize()
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    got = [[(torch.empty_like(src), torch.empty_like(src)) for src in x] for _ in range(6)]
+    torch.cuda.synchronize()
+    for rep in got:
+        for layer in (0, 1):
+            for m, s, src, (a, b) in zip(models, streams, x, rep):
+                with torch.cuda.stream(s):
+                    attention(m, layer, src if layer == 0 else a, a if layer == 0 else b)
+    torch.cuda.synchronize()
+    for rep in got:
+        for w, (_, b) in zip(want, rep):
+            assert torch.equal(b, w)
+    md.terminate_thread()
+    ops.check_device()
