@@ -471,9 +471,10 @@ bool plan_parts(const rt_encoder* e, int K, GemmPlan& plan) {
   const double rows = static_cast<double>(M) * N;
   const double parts_cost = plan.cost + (layernorm_parts_by_warps(M, N) ? 1.5 : 2.5) + rows * 6 / 6e6;
   double other;
-  if (N == 768) {  // LayerNorm is part of the cluster kernel's epilogue; 36 clusters of 128 rows, 22 of 256 are resident
-    if (M <= 36 * 128) other = 7.2 + K / 64 * 0.21 + M * 0.0007;
-    else other = 3.0 + ((M + 255) / 256 + 21) / 22 * (K / 64 * 0.32 + 3.6);
+  if (N == 768) {  // LayerNorm is part of the cluster kernel's epilogue: single CTAs while all row blocks are resident, or pairs
+    const int pairs = gemm_layernorm_clusters(N, true);
+    if (M <= gemm_layernorm_clusters(N, false) * 128) other = 7.2 + K / 64 * 0.21 + M * 0.0007;
+    else other = 3.0 + ((M + 255) / 256 + pairs - 1) / pairs * (K / 64 * 0.32 + 3.6);
   } else {
     other = plan_gemm(M, N, K, 1, false).cost + 1.9 + rows * 6 / 6e6;
   }
@@ -488,7 +489,7 @@ bool plan_parts(const rt_encoder* e, int K, GemmPlan& plan) {
 //   1024 columns, K = 4096 3072 rows 26.8 / 29.2  4096 44.2 / 31.6   12288 91.8 / 91.3  20480 141.5 / 152.0
 // 768-wide attention output, 12 layers, us, apart / fused: 3072 tokens 1055 / 1061, 3200 1053 / 1040, 5312 1347 / 1308,
 // 16384 3745 / 3649, 16512 3806 / 3712, 20352 4646 / 4596, 22656 5262 / 5177, 45312 9540 / 9330.
-// 1024-wide FFN down: 15 clusters of four pairs are resident, so 28 SMs idle.  From the second wave on that costs more than
+// 1024-wide FFN down: 15 clusters of four pairs are resident on 148 SMs, so 28 idle.  From the second wave on that costs more than
 // the LayerNorm until its traffic leaves L2, unless the projection alone needs as many waves of its 74 pairs (24 layers,
 // apart / fused: 4096 tokens 3315 / 3499, 4864 4028 / 4005, 8192 6078 / 6221, 10240 7494 / 7380, 11008 7991 / 7849).
 bool fuses_layernorm(const rt_encoder* e, int K) {
@@ -496,7 +497,10 @@ bool fuses_layernorm(const rt_encoder* e, int K) {
   if (N != 768 && N != 1024) return false;
   if (e->fuse_layernorm != 1) return e->fuse_layernorm == 2;
   if (N == 768) return K >= 2048 || blocks > 12;
-  return blocks > 10 && (K < 2048 || blocks > 48 || (blocks + 14) / 15 <= (blocks * 4 + 73) / 74);
+  if (blocks <= 10) return false;
+  if (K < 2048 || blocks > 48) return true;
+  const int clusters = gemm_layernorm_clusters(N, true), pairs = gemm_sm_count() / 2;
+  return (blocks + clusters - 1) / clusters <= (blocks * (N / 256) + pairs - 1) / pairs;
 }
 
 // The caller's pointers of a projection + LayerNorm.  The cluster kernel takes 32-byte aligned ones; a projection that

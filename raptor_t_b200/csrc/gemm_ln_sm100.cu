@@ -553,6 +553,11 @@ rt_status launch_ln(void* out, const void* a, const void* w, const void* bias, c
 }  // namespace rt
 
 namespace rt {
+int gemm_layernorm_clusters(int N, bool pairs) {
+  if (N == 768) return pairs ? resident_clusters<true, true, 3, 256>() : resident_clusters<true, false, 4, 192>();
+  return resident_clusters<true, true, 4, 256>();
+}
+
 rt_status gemm_layernorm_checked(void* out_dev, const void* a_dev, const void* w_dev, const void* bias_dev,
                                  const void* residual_dev, const void* gamma_dev, const void* beta_dev, int M, int N, int K,
                                  float eps, int dtype, void* stream, bool settled_w) {
@@ -577,7 +582,7 @@ rt_status gemm_layernorm_checked(void* out_dev, const void* a_dev, const void* w
   (bf ? launch_ln<true, PAIR, NT, TW>(out_dev, a_dev, w_dev, bias_dev, residual_dev, gamma_dev, beta_dev, M, K, eps, settled_w, st) \
       : launch_ln<false, PAIR, NT, TW>(out_dev, a_dev, w_dev, bias_dev, residual_dev, gamma_dev, beta_dev, M, K, eps, settled_w, st))
   if (N == 768) {
-    if (blocks <= resident_clusters<true, false, 4, 192>()) return RT_LN_LAUNCH(false, 4, 192);
+    if (blocks <= gemm_layernorm_clusters(N, false)) return RT_LN_LAUNCH(false, 4, 192);
     return RT_LN_LAUNCH(true, 3, 256);
   }
   return RT_LN_LAUNCH(true, 4, 256);

@@ -21,6 +21,11 @@ GemmPlan plan_gemm(int M, int N, int K, int max_splits, bool parts);
 rt_status run_gemm(void* c, const void* a, const void* w, const void* bias, int M, int N, int K, int epi, int dtype,
                    cudaStream_t st, const gemm_detail::QkvEpilogue& extra, const GemmPlan& plan);
 
+int gemm_sm_count();
+// Clusters of rt_gemm_bias_residual_layernorm that the current device keeps resident: of CTA pairs (256 rows), or of
+// single CTAs (128 rows, N = 768 only).  On a B200 22 and 36 for N = 768, 15 for N = 1024.
+int gemm_layernorm_clusters(int N, bool pairs);
+
 // rt_gemm, rt_gemm_bias_residual_layernorm and rt_gemm_qkv; settled_w as in QkvEpilogue.
 rt_status gemm_layernorm_checked(void* out, const void* a, const void* w, const void* bias, const void* residual,
                                  const void* gamma, const void* beta, int M, int N, int K, float eps, int dtype,
