@@ -28,6 +28,7 @@ kernel's own work list (pairs of query blocks per CTA) is built from the block t
 """
 import threading
 import time
+import weakref
 from concurrent.futures import ThreadPoolExecutor
 
 import numpy as np
@@ -123,15 +124,16 @@ class MetaData:
     """Per-batch kick of the metadata pipeline (layers/metadata.cpp:6-18).  Every
     registered attention layer gets a worker job that builds its block table and
     work list and uploads them; the layer waits for it right before its attention
-    kernel, after the QKV GEMM has been queued."""
-    _layers = []
+    kernel, after the QKV GEMM has been queued.  Layers are not kept alive: those of a model that is
+    gone are no longer planned for and their weights are free."""
+    _layers = []  # weak references
     _pool = None
     _lock = threading.Lock()
 
     @classmethod
     def register_layer(cls, layer):
         with cls._lock:
-            cls._layers.append(layer)
+            cls._layers = [r for r in cls._layers if r() is not None] + [weakref.ref(layer)]
 
     def update_meta_data(self, total_seq_len, to_select_index_len, to_select_index_position_len, seq_len_info):
         ts = TensorSet.get_instance()
@@ -140,7 +142,7 @@ class MetaData:
         if sum(lens) != int(total_seq_len):
             raise ValueError("update_meta_data: seq_len_info does not add up to total_seq_len")
         with MetaData._lock:
-            layers = list(MetaData._layers)
+            layers = [layer for layer in (r() for r in MetaData._layers) if layer is not None]
             if MetaData._pool is None:
                 MetaData._pool = ThreadPoolExecutor(max_workers=4, thread_name_prefix="raptor_meta")
         device = torch.cuda.current_device() if torch.cuda.is_available() else None

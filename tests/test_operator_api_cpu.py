@@ -31,6 +31,36 @@ def test_tensor_set_singleton_and_metadata_bookkeeping():
             pass
 
 
+def test_layers_of_a_model_that_is_gone_are_not_planned_for(monkeypatch):
+    import gc
+    import time
+    import weakref
+    w = torch.zeros(128, 384, dtype=torch.float16)
+    make = lambda i: raptor_t.BertAttention(w, w[0], w[:, :128], w[0, :128], w[0, :128], w[0, :128], 2, i, True)  # noqa: E731
+    planned = []
+    monkeypatch.setattr(raptor_t.BertAttention, "_build_plan", lambda self, lens, device: planned.append(self.layer_idx))
+    md = raptor_t.MetaData()
+    kept, gone = [make(0), make(1)], [make(2), make(3)]
+    md.update_meta_data(512, 9, 64, [0, 8])
+    for layer in kept + gone:
+        layer._pending.result()
+    assert sorted(planned) == [0, 1, 2, 3]
+    dead = [weakref.ref(layer) for layer in gone]
+    del gone, layer
+    for _ in range(500):  # a worker lets go of its job a moment after the result is there
+        gc.collect()
+        if all(r() is None for r in dead):
+            break
+        time.sleep(0.01)
+    assert all(r() is None for r in dead)
+    planned.clear()
+    md.update_meta_data(512, 9, 64, [0, 8])
+    for layer in kept:
+        layer._pending.result()
+    assert sorted(planned) == [0, 1]
+    md.terminate_thread()
+
+
 def test_compiled_module_exports_the_reference_classes():
     """The pybind11 module `raptor_t` builds, imports without a GPU and carries every class and
     method of the reference's extension module (python/pybind.cpp:11-80)."""
