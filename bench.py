@@ -268,7 +268,7 @@ def run_gpu(args, w):
         if h2d:
             b.ids_dev.copy_(b.ids_pinned, non_blocking=True)
         out = out_devs[k][: b.T_local]
-        # host work of the step: metadata hand-off + ~90 kernel launches, without the time the thread sits
+        # host work of the step: metadata hand-off + the kernel launches, without the time the thread sits
         # waiting for the GPU to release a metadata slot (it runs ahead of the GPU until the slots are used up)
         t0, blocked0 = time.perf_counter(), enc.host_blocked_ms()
         enc.prepare(b.lens)

@@ -89,8 +89,9 @@ __device__ __forceinline__ float warp_sum(float v) {
 // registers and many warps (loads in flight) per SM.
 // Bound by HBM as long as loads are in flight all the time: a row's 16-bit vectors are on their way while the warp
 // reduces, normalises and stores the one before (32768 rows from HBM, 768 columns 26.8 -> 25.4 us = 5.9 TB/s, a plain
-// copy of the same traffic 26.6; 1024 columns 35.8 -> 32.2, 2048 columns 76.7 -> 63.7).  CTAs per SM as registers allow without spills: 1024 columns
-// with three 34.0 us.
+// copy of the same traffic 26.6; 1024 columns 35.8 -> 32.2, 2048 columns 76.7 -> 63.7; below one row per warp up to 0.1 us
+// slower: 2400 rows of 64 columns 1.79 -> 1.88).  CTAs per SM as registers allow without spills: 1024 columns with three
+// 34.0 us.
 // ---------------------------------------------------------------------------
 constexpr int layernorm_ctas(int nv) { return nv <= 3 ? 3 : nv <= 6 ? 2 : 1; }  // resident per SM
 template <typename T, int NV>

@@ -6,13 +6,13 @@
 // the per-layer std::async workers of layers/multi_headed_attention.h:72-110 on
 // CUDA streams and events): the encoder owns ONE persistent host worker.
 // prepare_batch() hands it the batch; it builds, layer by layer, the attention work
-// list into pinned memory, enqueues one upload per layer on a side stream and records
-// an event per layer.  Query-block pairs, cuts of long lists and the assignment of
+// list into pinned memory, enqueues one upload per layer (one for all layers where
+// their lists are short) on a side stream and records an event behind each.  Query-block pairs, cuts of long lists and the assignment of
 // work items to CTAs are computed once per batch (layer 0); the other layers only
 // refill the list entries from their own block tables.  The forward pass issues the
-// QKV GEMM of layer i first, then makes the compute stream wait on layer i's event
-// (after a host-side check that the event has been recorded), so table construction
-// and upload overlap the GEMMs.
+// QKV GEMM of layer i first, then makes the compute stream wait for the upload that
+// holds layer i's list (after a host-side check that its event has been recorded), so
+// table construction and upload overlap the GEMMs.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -641,6 +641,8 @@ rt_status run_output(rt_encoder* e, int l, const void* ffn, const void* residual
     return RT_OK;
   }
   {
+    // weights not requested ahead: no difference (12 layers of 1024 columns, plain / ahead: 4096 tokens 1451 / 1452 us, 4608
+    // 1542 / 1545, 9472 3062 / 3063)
     Span s(e, st, "gemm.ffn_down");
     RT_TRY(rt_gemm(dense, ffn, w.down_w.p, nullptr, e->tokens, c.hidden, c.ffn, RT_EPI_NONE, c.dtype, st));
   }

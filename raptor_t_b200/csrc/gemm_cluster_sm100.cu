@@ -31,7 +31,8 @@ using namespace ptx;
 using namespace gemm_detail;
 
 constexpr int kBM = 128, kBN = 64, kBK = 64;
-constexpr int kStages = 6;  // all K blocks of a CTA for K <= 768; one CTA per SM (two, with 3 stages, were packed onto half of the SMs)
+// All K blocks of a CTA for K <= 768; one CTA per SM (two, with 3 stages, were packed onto half of the SMs).
+constexpr int kStages = 6;
 constexpr int kABytes = kBM * kBK * 2;
 constexpr int kWBytes = kBN * kBK * 2;
 constexpr int kStageBytes = kABytes + kWBytes;

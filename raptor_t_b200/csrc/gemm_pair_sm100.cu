@@ -258,8 +258,9 @@ rt_status launch_pair(void* c, const void* a, const void* w, const void* bias, i
   const int mn = main_tiles + ((M + kTileM - 1) / kTileM) * (N / tail_w) - (main_tiles ? main_tiles * (kTileN / tail_w) : 0);
   const int tiles = mn * (EPI == kEpiPartial ? qkv.splits : 1);
   const int pairs = std::min(tiles, sms / 2);
-  // Only where the launch fills the chip.  12 layers: 4096 tokens 1177 -> 1173 us, 5312 1279 -> 1272, 1024 wide (24 layers) 4096
-  // tokens 3462 -> 3421; with CTAs that wait on free SMs for longer, 256 tokens 435 -> 437, 1024 wide 1024 tokens 1544 -> 1550.
+  // Only where the launch fills the chip.  12 layers: 4096 tokens 1177 -> 1173 us, 5312 1279 -> 1272, 1024 wide (24
+  // layers) 4096 tokens 3462 -> 3421; with CTAs that wait on free SMs for longer, 256 tokens 435 -> 437, 1024 wide 1024
+  // tokens 1544 -> 1550.
   QkvEpilogue args = qkv;
   args.settled_w = qkv.settled_w && pairs == sms / 2;
   RT_CHECK_CUDA(launch_kernel(kern, dim3(2 * pairs), dim3(kThreads), kSmemBytes, st, ma, mw, mwt, mc, mk, mv, main_tiles, tail_w, (uint16_t*)c,

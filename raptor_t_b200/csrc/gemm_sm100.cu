@@ -56,8 +56,8 @@ constexpr int kEpilogueThreads = 256;  // two warps per TMEM lane quarter, alter
 // below that, narrower tiles on more SMs are faster (768 columns, K = 3072, 4096 rows: 48 pair tiles of 256
 // columns 19.9 us, 64 of 192 15.9 us, 192 single-CTA tiles of 128 25.1 us).  For as many waves of 256 columns the
 // pairs stay ahead: alone, us, single CTAs / pairs, 1024 columns: 3840 rows K = 4096 29.5 / 26.8, 5120 33.1 / 30.9, 8192
-// 54.6 / 49.7, 4454 rows K = 4096 31.0 / 28.8.  Up to K = 2048 single CTAs are faster alone (K = 1024, 3840 rows 9.6 / 10.5) but not in
-// the chain of a forward, where pairs start earlier (12 layers of 1024 columns, 1024 tokens, FFN up 781 / 775, 1536, QKV 930 / 922).
+// 54.6 / 49.7, 4454 rows K = 4096 31.0 / 28.8.  Up to K = 2048 single CTAs are faster alone (K = 1024, 3840 rows 9.6 / 10.5)
+// but not in the chain of a forward (12 layers of 1024 columns: FFN up of 1024 tokens 781 / 775, QKV of 1536 930 / 922).
 struct TileCost {
   int width;
   double launch, k_block, tile;

@@ -1,6 +1,6 @@
 // Kernel launch with programmatic dependent launch: the next kernel in the stream may be
 // scheduled (and run its prologue up to griddepcontrol.wait) while the previous one drains,
-// which hides most of the launch latency between the ~90 dependent kernels of a forward pass.
+// which hides most of the launch latency between the 62 to 110 dependent kernels of a forward pass.
 #pragma once
 #include <cuda_runtime.h>
 

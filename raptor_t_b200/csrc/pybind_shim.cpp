@@ -318,9 +318,9 @@ PlanResult build_plan(const rt_config& c, uint32_t seed, const std::vector<int32
 
 // The work list of one batch for all layers with the same block lists: the same model constants, and the same layer
 // index where a sequence is long enough for random blocks.  A program with several models has 12 layers of each
-// registered, whichever of them the batch is for: 6464 tokens with three 12-layer models alive 3764 us a batch with a task per
-// layer, 1784 with one per list (with one model alive 1773).  The partial results of cut lists are part of it: the calls of all layers
-// are ordered on the device (SharedUse).
+// registered, whichever of them the batch is for: 6464 tokens with three 12-layer models alive 3764 us a batch with a
+// task per layer, 1784 with one per list; with one model alive 1773 either way.  The partial results of cut lists are part
+// of it: the calls of all layers are ordered on the device (SharedUse).
 class BatchPlan {
  public:
   using Key = std::array<int64_t, 9>;
